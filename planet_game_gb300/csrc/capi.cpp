@@ -10,6 +10,7 @@
 
 #include "column.hpp"
 #include "host/insolation.hpp"
+#include "onchip_plan.hpp"
 #include "operators.hpp"
 #include "profile.hpp"
 #include "solver.hpp"
@@ -971,6 +972,7 @@ int psgb_batch_set_priority(psgb_batch* h, int high) {
         PSGB_CUDA(cudaStreamCreateWithPriority(&fresh, cudaStreamNonBlocking, high != 0 ? greatest : least));
         PSGB_CUDA(cudaStreamSynchronize(b.stream));
         PSGB_CUDA(cudaStreamDestroy(b.stream));
+        b.onchip.clear();   // their streams have the old priority
         b.stream = fresh;
         return PSGB_OK;
     });

@@ -1,0 +1,11 @@
+// The on-chip solves in FP64: see onchip_kernel.cuh.
+#include "onchip_kernel.cuh"
+
+namespace psgb {
+
+template unsigned onchip_shared_limit<double>(int);
+template unsigned onchip_max_threads<double>(int);
+template int onchip_active_clusters<double>(int, unsigned, unsigned, std::size_t);
+template void onchip_launch<double>(const OnchipArgs<double>&, int, unsigned, std::size_t, cudaStream_t);
+
+}  // namespace psgb

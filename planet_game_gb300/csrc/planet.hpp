@@ -201,6 +201,8 @@ struct GraphEntry {
     std::uint64_t kernels = 0;
 };
 
+struct OnchipPlan;   // onchip_plan.hpp
+
 struct SmootherConfig {
     int pre = 2, post = 2;             // damped Jacobi sweeps on every level ...
     double omega = 0.8;                // damping factor
@@ -276,6 +278,8 @@ struct Batch {
     cudaEvent_t fence_in = nullptr, fence_out = nullptr;
     std::map<GraphKey, GraphEntry> graphs;
     bool use_graphs = true;
+    // on-chip solves: per precision and block-local levels, which planets and how
+    std::map<std::vector<int>, std::unique_ptr<OnchipPlan>> onchip;
     // transport-step buffers (fine layout)
     double* slope_of = nullptr;        // [instances] dt / C
     double* t0 = nullptr;              // [P0]
@@ -298,13 +302,8 @@ struct Batch {
     std::vector<std::vector<double>> stored_edges;      // per planet: set with psgb_batch_set_edge_conductance
     std::vector<std::uint64_t> stored_generation;       // per planet: bumped on every set
     std::uint64_t assembled_bytes_hint = 0;
-    ~Batch() {
-        for (auto& g : graphs) cudaGraphExecDestroy(g.second.exec);
-        if (fence_in != nullptr) cudaEventDestroy(fence_in);
-        if (fence_out != nullptr) cudaEventDestroy(fence_out);
-        if (stream != nullptr) cudaStreamDestroy(stream);
-        if (pinned_scalars != nullptr) cudaFreeHost(pinned_scalars);
-    }
+    Batch();
+    ~Batch();
 };
 
 }  // namespace psgb

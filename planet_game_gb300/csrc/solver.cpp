@@ -13,6 +13,7 @@
 #include "host/agglomerate.hpp"
 #include "host/shared_columns.hpp"
 #include "krylov.hpp"
+#include "onchip_plan.hpp"
 #include "persistent.hpp"
 #include "profile.hpp"
 
@@ -23,6 +24,16 @@
 #include <stdexcept>
 
 namespace psgb {
+
+Batch::Batch() = default;
+
+Batch::~Batch() {
+    for (auto& g : graphs) cudaGraphExecDestroy(g.second.exec);
+    if (fence_in != nullptr) cudaEventDestroy(fence_in);
+    if (fence_out != nullptr) cudaEventDestroy(fence_out);
+    if (stream != nullptr) cudaStreamDestroy(stream);
+    if (pinned_scalars != nullptr) cudaFreeHost(pinned_scalars);
+}
 
 namespace {
 
@@ -957,6 +968,17 @@ bool use_persistent(const Batch& b, const SolveOptions& opt) {
     return true;
 }
 
+// The on-chip solves of the automatic schedule: BiCGSTAB on planets that fit a cluster. A
+// tuning that asks for a coarse tail, a recording profile (whose families are the kernel
+// schedule's) and a batch on its caller's stream keep the kernel schedule.
+OnchipPlan* onchip_for(Batch& b, const SolveOptions& opt) {
+    if (opt.schedule != kScheduleAuto || opt.method != kBiCGSTAB || b.stream == nullptr || profile_active() ||
+        (b.tuned && b.tail_level > 0))
+        return nullptr;
+    OnchipPlan& plan = opt.precision == kMixed ? onchip_plan<float>(b) : onchip_plan<double>(b);
+    return plan.classes.empty() ? nullptr : &plan;
+}
+
 }  // namespace
 
 void solve(Batch& b, const SolveOptions& opt, const double* rhs, double* x, cudaStream_t caller) {
@@ -971,10 +993,14 @@ void solve(Batch& b, const SolveOptions& opt, const double* rhs, double* x, cuda
     const LevelView<double> lv64 = view64(b, 0);
     const ReduceCtx ctx = reduce_ctx(b);
     const bool persistent = use_persistent(b, opt);
+    OnchipPlan* const plan = onchip_for(b, opt);
     // Inner target: max(inner_tol * ||r||, tolerance * ||b|| / 2); the plain FP64 solve
     // reaches the outer target in one refinement, the mixed one in a few.
     const double inner_tol = opt.precision == kMixed ? opt.inner_tolerance : 1e-3 * opt.tolerance;
-    if (!persistent) {
+    if (plan != nullptr) {
+        if (opt.precision == kMixed) onchip_solve<float>(b, *plan, opt, rhs, x, inner_tol, st);
+        else onchip_solve<double>(b, *plan, opt, rhs, x, inner_tol, st);
+    } else if (!persistent) {
         launch_outer_init(lv64, rhs, ctx, opt.tolerance, opt.max_refinements, b.active_mask ? b.active : nullptr, st);
     } else {
         // The whole refinement loop in one cooperative launch (outer_init included).
@@ -985,7 +1011,7 @@ void solve(Batch& b, const SolveOptions& opt, const double* rhs, double* x, cuda
             launch_persistent<double>(persistent_args<double>(b, opt, rhs, x, inner_tol), st, b.stream != nullptr);
         }
     }
-    for (int refine = 0; !persistent && refine <= opt.max_refinements; ++refine) {
+    for (int refine = 0; !persistent && plan == nullptr && refine <= opt.max_refinements; ++refine) {
         if (opt.precision == kMixed) {
             launch_outer_residual<float>(lv64, rhs, x, b.rr, b.k32[8], ctx, opt.max_refinements, st);
         } else {
@@ -1003,7 +1029,7 @@ void solve(Batch& b, const SolveOptions& opt, const double* rhs, double* x, cuda
     InstanceScalars* host = b.pinned_scalars != nullptr ? b.pinned_scalars : b.host_scalars.data();
     PSGB_CUDA(cudaMemcpyAsync(host, b.scalars, b.instances * sizeof(InstanceScalars), cudaMemcpyDeviceToHost, st));
     unsigned barrier_error[2] = {0, 0};
-    const TailForm form = persistent ? TailForm::kNone
+    const TailForm form = persistent || plan != nullptr ? TailForm::kNone
                                      : (opt.precision == kMixed ? tail_form<float>(b) : tail_form<double>(b));
     if (persistent || form == TailForm::kSpread || form == TailForm::kCluster) {
         PSGB_CUDA(cudaMemcpyAsync(barrier_error, b.sync + 2, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, st));

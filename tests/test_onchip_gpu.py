@@ -1,0 +1,95 @@
+"""The on-chip solves (one planet per thread-block cluster) against the kernel schedule: the
+same phases and reduction trees, so every result is the same bits - planets alone and in
+batches, left-out planets, every precision, sweep setting and ending of the iteration."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def inputs_of(mesh, seed):
+    from planet_game_gb300 import workloads as W
+
+    return W.step_inputs(mesh, seed=seed, edge_diffusivity=W.lognormal_edge_diffusivity(mesh.edge_count, 300 + seed))
+
+
+def step(batch, inputs, **options):
+    keep = options.pop("keep", range(len(inputs)))
+    pick = lambda f: [f(i) if k in keep else None for k, i in enumerate(inputs)]
+    active = [k in keep for k in range(len(inputs))]
+    return batch.transport_step(pick(lambda i: i.t0), pick(lambda i: i.source), 4e7, inputs[0].dt,
+                                edge_conductance=[i.edge_conductance for i in inputs],
+                                active=None if all(active) else active, **options)
+
+
+def same(a, b):
+    (out_a, rep_a), (out_b, rep_b) = a, b
+    for x, y in zip(out_a, out_b):
+        assert (x is None) == (y is None)
+        assert x is None or np.array_equal(x, y)
+    for x, y in zip(rep_a, rep_b):
+        assert (x.status, x.refinements, x.iterations) == (y.status, y.refinements, y.iterations)
+        assert x.relative_residual == y.relative_residual
+
+
+# levels 3 (two levels, 42 coarsest rows) to 6 (the largest that fits a cluster in FP32)
+@pytest.mark.parametrize("level,precision", [(3, "fp64"), (3, "mixed"), (4, "fp64"), (4, "mixed"), (5, "fp64"),
+                                             (5, "mixed"), (6, "mixed"), (6, "fp64")])
+def test_one_planet_equals_the_kernel_schedule(meshes, level, precision):
+    import planet_game_gb300 as pg
+
+    m = meshes(level, 3.4e6)
+    batch, inputs = pg.Batch([m]), [inputs_of(m, level)]
+    for options in ({}, {"pre_sweeps": 1, "post_sweeps": 1, "jacobi_omega": 1.0}, {"pre_sweeps": 1, "post_sweeps": 0},
+                    {"pre_sweeps": 3, "post_sweeps": 2}, {"max_iterations": 2, "max_refinements": 3},
+                    {"tolerance": 1e-3}):
+        same(step(batch, inputs, precision=precision, **options),
+             step(batch, inputs, precision=precision, schedule="kernels", **options))
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_batches_of_several_levels(meshes, precision):
+    """Several sizes of cluster side by side, and a batch that one planet keeps off chip; some
+    planets left out of the step."""
+    import planet_game_gb300 as pg
+
+    for levels in ((5, 3, 4, 5, 4), (5, 3, 7, 4, 5)):
+        ms = [meshes(l, 3.0e6 + 0.4e6 * i) for i, l in enumerate(levels)]
+        inputs = [inputs_of(m, i) for i, m in enumerate(ms)]
+        batch = pg.Batch(ms)
+        for keep in (range(5), (0, 2), (1, 4), (2,)):
+            same(step(batch, inputs, precision=precision, keep=keep),
+                 step(batch, inputs, precision=precision, keep=keep, schedule="kernels"))
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_tuned_sweeps(meshes, precision):
+    """Block-local coarse sweeps (whole tiles per block) and a scaled coarse correction."""
+    import planet_game_gb300 as pg
+
+    ms = [meshes(l, 3.2e6 + 0.3e6 * i) for i, l in enumerate((5, 6, 4, 5, 3))]
+    inputs = [inputs_of(m, 20 + i) for i, m in enumerate(ms)]
+    batch = pg.Batch(ms)
+    depth = batch.tuning["levels"]
+    for inner, correction, omega in ((6, 1.0, 1.0), (3, 2.0, 0.9), (1, 1.5, 0.8)):
+        batch.set_tuning({"pre_sweeps": [1] + [2] * (depth - 1), "post_sweeps": [1] + [2] * (depth - 1),
+                          "stencil_tiles": [1] * depth, "vector_tiles": [1] * depth,
+                          "block_sweeps": [1] + [inner] * (depth - 1), "jacobi_omega": omega,
+                          "coarse_correction": correction})
+        same(step(batch, inputs, precision=precision), step(batch, inputs, precision=precision, schedule="kernels"))
+
+
+def test_non_finite_source_reports_and_keeps_the_other_planets(meshes):
+    import planet_game_gb300 as pg
+
+    ms = [meshes(4, 3.3e6), meshes(5, 4.1e6)]
+    inputs = [inputs_of(m, 40 + i) for i, m in enumerate(ms)]
+    bad = inputs[0].source.copy()
+    bad[7] = np.nan
+    batch = pg.Batch(ms)
+    args = lambda s0: ([i.t0 for i in inputs], [s0, inputs[1].source], 4e7, inputs[0].dt)
+    edges = [i.edge_conductance for i in inputs]
+    good = batch.transport_step(*args(inputs[0].source), edge_conductance=edges, precision="mixed")
+    with pytest.raises(Exception, match="non-finite"):
+        batch.transport_step(*args(bad), edge_conductance=edges, precision="mixed")
+    same(good, batch.transport_step(*args(inputs[0].source), edge_conductance=edges, precision="mixed"))
