@@ -106,10 +106,12 @@ void tune_shapes(Batch& b, cudaStream_t st) {
     int pick = b.tail_level;
     for (int tail = 0; tail < static_cast<int>(b.levels.size()); ++tail) {
         b.tail_level = tail;
+        b.tail_auto = tail == 0;
         const double ms = time_launches(st, [&] { vcycle<T>(b, rhs, x, kGateAlways, false, st); });
         if (best < 0.0 || ms < best) { best = ms; pick = tail; }
     }
     b.tail_level = pick;
+    b.tail_auto = pick == 0;
     PSGB_CUDA(cudaGetLastError());
 }
 
@@ -210,6 +212,7 @@ void apply_tuning(Batch& b, const Tuning& t) {
     b.smoother.omega = t.omega;
     b.smoother.correction = t.correction;
     b.tail_level = t.tail_level;
+    b.tail_auto = t.tail_level == 0;
     b.tail_spread = t.tail_spread;
     b.tail_shared = t.tail_shared;
     b.tail_cluster = t.tail_cluster;
@@ -367,12 +370,14 @@ Tuning autotune(Batch& b, const SolveOptions& opt, const double* rhs, const doub
                                          : tail_fits_cluster<double>(b, tail, cluster)))
                     continue;
                 b.tail_level = tail;
+                b.tail_auto = tail == 0;
                 set_mode(mode);
                 const double ms = run(best);
                 if (ms > 0.0 && ms < best_ms) { best_ms = ms; pick = tail; pick_mode = mode; }
             }
         }
         b.tail_level = pick;
+        b.tail_auto = pick == 0;
         set_mode(pick_mode);
     }
     // the fine level's tile-set sizes again, by whole solves with everything else chosen: a

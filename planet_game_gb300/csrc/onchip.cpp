@@ -27,17 +27,11 @@ template <>
 struct Pick<double> {
     static LevelView<double> view(const Batch& b, std::size_t l) { return view64(b, l); }
     static const double* inv(const DenseCoarse& D) { return D.inv64; }
-    static double* x(BatchLevel& L) { return L.x64; }
-    static double* y(BatchLevel& L) { return L.y64; }
-    static double* bvec(BatchLevel& L) { return L.b64; }
 };
 template <>
 struct Pick<float> {
     static LevelView<float> view(const Batch& b, std::size_t l) { return view32(b, l); }
     static const float* inv(const DenseCoarse& D) { return D.inv32; }
-    static float* x(BatchLevel& L) { return L.x32; }
-    static float* y(BatchLevel& L) { return L.y32; }
-    static float* bvec(BatchLevel& L) { return L.b32; }
 };
 
 std::uint32_t ceil_div(std::uint32_t a, std::uint32_t b) { return (a + b - 1) / b; }
@@ -61,10 +55,10 @@ std::uint32_t members_most(const HostLevel& fine, std::uint32_t coarse_rows, std
     return *std::max_element(held.begin(), held.end());
 }
 
-// Shared-memory layout of levels [first, coarsest]; returns the bytes, and the offsets in
+// Shared-memory layout of a block; returns the bytes, and the offsets in
 // `a` when it is given.
 template <typename T>
-std::size_t layout(const OnchipClass& c, int first, OnchipArgs<T>* a) {
+std::size_t layout(const OnchipClass& c, OnchipArgs<T>* a) {
     std::size_t at = 0, o_r0 = 0;
     const auto take = [&](std::size_t bytes) {
         const std::size_t o = at;
@@ -72,7 +66,7 @@ std::size_t layout(const OnchipClass& c, int first, OnchipArgs<T>* a) {
         return static_cast<std::uint32_t>(o);
     };
     const int coarsest = static_cast<int>(c.rows.size()) - 1;
-    for (int l = first; l <= coarsest; ++l) {
+    for (int l = 0; l <= coarsest; ++l) {
         OnchipLevel<T> scratch{};
         OnchipLevel<T>& L = a != nullptr ? a->level[l] : scratch;
         const std::size_t span = c.span[l];
@@ -86,7 +80,7 @@ std::size_t layout(const OnchipClass& c, int first, OnchipArgs<T>* a) {
             L.o_moff = take(std::size_t(c.span[l + 1]) * 4);
             L.o_mem = take(std::size_t(c.members[l]) * 4);
             L.o_r = take(span * sizeof(T));
-            if (l == first) o_r0 = L.o_r;
+            if (l == 0) o_r0 = L.o_r;
             L.o_y = take(span * sizeof(T));
         }
         if (l > 0) {
@@ -95,15 +89,15 @@ std::size_t layout(const OnchipClass& c, int first, OnchipArgs<T>* a) {
         }
     }
     const std::size_t dense = take(std::size_t(c.span[coarsest]) * c.rows[coarsest] * sizeof(T));
-    const std::size_t phat = first == 0 ? take(c.span[0] * sizeof(T)) : 0;
-    const std::size_t shat = first == 0 ? take(c.span[0] * sizeof(T)) : 0;
+    const std::size_t phat = take(c.span[0] * sizeof(T));
+    const std::size_t shat = take(c.span[0] * sizeof(T));
     // every 32-row partial of the planet, two quantities in T or one in FP64, two sets in turn;
     // the second lies where the fine residual does when it fits there (a V-cycle's phases all
     // lie between two reductions)
-    const std::size_t part_bytes = std::size_t(ceil_div(c.rows[first], 256u)) * 8 * std::max(2 * sizeof(T), sizeof(double));
-    const std::size_t part = first == 0 ? take(part_bytes) : 0;
+    const std::size_t part_bytes = std::size_t(ceil_div(c.rows[0], 256u)) * 8 * std::max(2 * sizeof(T), sizeof(double));
+    const std::size_t part = take(part_bytes);
     std::size_t part2 = o_r0;
-    if (first == 0 && part_bytes > c.span[0] * sizeof(T)) part2 = take(part_bytes);
+    if (part_bytes > c.span[0] * sizeof(T)) part2 = take(part_bytes);
     const std::size_t list = take(std::size_t(c.phases) * kOnchipPhaseBytes);
     if (a != nullptr) {
         a->o_list = static_cast<std::uint32_t>(list);
@@ -117,21 +111,21 @@ std::size_t layout(const OnchipClass& c, int first, OnchipArgs<T>* a) {
 }
 
 // Spans and member bounds for a cluster size; false where a level cannot be held so.
-bool spread(const Batch& b, OnchipClass& c, unsigned cluster, int first) {
+bool spread(const Batch& b, OnchipClass& c, unsigned cluster) {
     const std::size_t depth = c.rows.size();
     c.cluster = cluster;
     c.phases = 1;
-    for (std::size_t l = first; l + 1 < depth; ++l) c.phases += b.smoother.pre_at(l) + b.smoother.post_at(l) + 2;
+    for (std::size_t l = 0; l + 1 < depth; ++l) c.phases += b.smoother.pre_at(l) + b.smoother.post_at(l) + 2;
     if (c.phases > kOnchipMaxPhases) return false;
     c.span.assign(depth, 0);
     c.members.assign(depth, 0);
-    for (std::size_t l = first; l < depth; ++l) {
-        const bool leading = l == static_cast<std::size_t>(first);
-        c.span[l] = span_of(c.rows[l], cluster, leading, l + 1 < depth && b.smoother.inner_at(l) > 1,
-                            leading ? 1.0 : static_cast<double>(c.span[first]) / c.rows[first]);
+    for (std::size_t l = 0; l < depth; ++l) {
+        const bool fine = l == 0;
+        c.span[l] = span_of(c.rows[l], cluster, fine, l + 1 < depth && b.smoother.inner_at(l) > 1,
+                            fine ? 1.0 : static_cast<double>(c.span[0]) / c.rows[0]);
         if (c.span[l] > kOnchipMaxSpan || (l + 1 < depth && b.levels[l].width > 8)) return false;
     }
-    for (std::size_t l = first; l + 1 < depth; ++l) {
+    for (std::size_t l = 0; l + 1 < depth; ++l) {
         for (std::uint32_t i : c.planets)
             c.members[l] = std::max(c.members[l], members_most(b.planets[i]->hierarchy.levels[l], c.rows[l + 1], c.span[l + 1]));
     }
@@ -155,7 +149,7 @@ void choose(const Batch& b, OnchipClass& c) {
     for (unsigned cluster : {1u, 2u, 4u, 8u, 16u}) {
         if (!fits) break;
         OnchipClass t = c;
-        if (!spread(b, t, cluster, 0)) continue;
+        if (!spread(b, t, cluster)) continue;
         // block-local sweeps: a block's threads hold all of its coarse rows, or whole tiles of them
         std::uint32_t local = 0;
         for (std::size_t l = 1; l + 1 < c.rows.size(); ++l)
@@ -164,10 +158,10 @@ void choose(const Batch& b, OnchipClass& c) {
             t.rows_per_thread = r;
             t.threads = std::max(256u, ceil_div(ceil_div(t.span[0], static_cast<std::uint32_t>(r)), 32u) * 32u);
             if (local > t.threads) t.threads = ceil_div(t.threads, 256u) * 256u;
-            if (t.threads <= onchip_max_threads<T>(r)) break;
+            if (t.threads <= kOnchipThreads) break;
         }
-        if (t.threads > onchip_max_threads<T>(t.rows_per_thread)) continue;
-        t.shared_bytes = layout<T>(t, 0, static_cast<OnchipArgs<T>*>(nullptr));
+        if (t.threads > kOnchipThreads || !onchip_has<T>(t.rows_per_thread)) continue;
+        t.shared_bytes = layout<T>(t, static_cast<OnchipArgs<T>*>(nullptr));
         const int active = onchip_active_clusters<T>(t.rows_per_thread, cluster, t.threads, t.shared_bytes);
         if (active <= 0) continue;
         const double waves = ceil_div(static_cast<std::uint32_t>(c.planets.size()), static_cast<std::uint32_t>(active));
@@ -222,6 +216,7 @@ OnchipPlan& onchip_plan(Batch& b) {
     if (!fits || std::max(longest, shared) > launch) plan->classes.clear();
     for (std::size_t k = 0; k < plan->classes.size(); ++k) {
         OnchipClass& c = plan->classes[k];
+        if (plan->classes.size() == 1) break;   // every planet of the batch, in its order
         PSGB_CUDA(cudaMalloc(reinterpret_cast<void**>(&c.list), c.planets.size() * sizeof(std::uint32_t)));
         PSGB_CUDA(cudaMemcpy(c.list, c.planets.data(), c.planets.size() * sizeof(std::uint32_t), cudaMemcpyHostToDevice));
         if (k == 0) continue;
@@ -243,10 +238,10 @@ OnchipPlan& onchip_plan(Batch& b) {
 namespace {
 
 template <typename T>
-OnchipArgs<T> arguments(Batch& b, const OnchipClass& c, int first) {
+OnchipArgs<T> arguments(Batch& b, const OnchipClass& c) {
     OnchipArgs<T> a{};
     const int coarsest = static_cast<int>(c.rows.size()) - 1;
-    for (int l = first; l <= coarsest; ++l) {
+    for (int l = 0; l <= coarsest; ++l) {
         BatchLevel& L = b.levels[static_cast<std::size_t>(l)];
         const LevelView<T> v = Pick<T>::view(b, static_cast<std::size_t>(l));
         OnchipLevel<T>& o = a.level[l];
@@ -256,9 +251,6 @@ OnchipArgs<T> arguments(Batch& b, const OnchipClass& c, int first) {
         o.agg = L.agg;
         o.moff = L.member_offset;
         o.member = L.member;
-        o.gx = Pick<T>::x(L);
-        o.gy = Pick<T>::y(L);
-        o.gb = Pick<T>::bvec(L);
         o.pitch = L.rows;
         o.width = L.width;
         o.n = c.rows[static_cast<std::size_t>(l)];
@@ -269,7 +261,6 @@ OnchipArgs<T> arguments(Batch& b, const OnchipClass& c, int first) {
         o.starts_in_x = b.smoother.starts_in_x(l) ? 1 : 0;
         o.correction = v.correction;
     }
-    a.first = first;
     a.coarsest = coarsest;
     a.cluster = static_cast<int>(c.cluster);
     a.planets = static_cast<std::uint32_t>(c.planets.size());
@@ -280,7 +271,7 @@ OnchipArgs<T> arguments(Batch& b, const OnchipClass& c, int first) {
     a.dense_inv = Pick<T>::inv(b.dense);
     a.omega = static_cast<T>(b.smoother.omega);
     a.sc = b.scalars;
-    layout<T>(c, first, &a);
+    layout<T>(c, &a);
     return a;
 }
 
@@ -292,7 +283,7 @@ void onchip_solve(Batch& b, OnchipPlan& plan, const SolveOptions& opt, const dou
     if (!plan.streams.empty()) PSGB_CUDA(cudaEventRecord(plan.fork, st));
     for (std::size_t k = 0; k < plan.classes.size(); ++k) {
         const OnchipClass& c = plan.classes[k];
-        OnchipArgs<T> a = arguments<T>(b, c, 0);
+        OnchipArgs<T> a = arguments<T>(b, c);
         a.fine_col = b.levels[0].col;
         a.fine_vd64 = b.levels[0].vd64;
         a.rhs64 = rhs;

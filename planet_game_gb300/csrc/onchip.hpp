@@ -1,9 +1,7 @@
 // Solves held on chip: one planet per thread-block cluster, its matrix hierarchy and every
 // vector of the solve spread over the shared memory and registers of the cluster's blocks.
 //
-// Two kernels share the layout (onchip_kernel.cuh):
-//   k_onchip_solve  a whole refined BiCGSTAB solve of one planet in one launch;
-//   k_onchip_cycle  the coarse levels of one V-cycle of a planet too large for that.
+// k_onchip_solve (onchip_kernel.cuh) runs a whole refined BiCGSTAB solve in one launch.
 // Arguments are plain device pointers, sizes and shared-memory offsets, filled by the host
 // driver (onchip.cpp).
 #pragma once
@@ -31,9 +29,6 @@ struct OnchipLevel {
     const std::int32_t* agg;   // [pitch]: row on the next level (absent on the coarsest)
     const std::uint32_t* moff; // next level's member lists
     const std::uint32_t* member;
-    T* gx;                     // k_onchip_cycle, its first level: the batch's iterate
-    T* gy;                     // ... ping-pong partner and right-hand side
-    T* gb;
     std::uint32_t pitch;
     std::uint32_t width;       // ELL width: 6 or 8
     std::uint32_t n;           // rows of each planet of the launch
@@ -48,11 +43,11 @@ struct OnchipLevel {
 template <typename T>
 struct OnchipArgs {
     OnchipLevel<T> level[kMaxLevels];
-    int first, coarsest;                // levels held (first > 0: the cycle kernel)
+    int coarsest;                       // the last level
     int cluster;                        // blocks per planet
     std::uint32_t planets;              // planets of the launch
     std::uint32_t instances;            // planets of the batch
-    const std::uint32_t* list;          // [planets] their indices in the batch
+    const std::uint32_t* list;          // [planets] their indices in the batch (null: 0, 1, ...)
     const std::uint32_t* tile_range;    // [levels][instances][2]
     const std::uint64_t* dense_offset;  // per planet, into dense_inv
     const T* dense_inv;
@@ -60,8 +55,6 @@ struct OnchipArgs {
     std::uint32_t o_part2;              // reductions' partials alternate between o_part and here
     T omega;
     InstanceScalars* sc;
-    int gate;                           // k_onchip_cycle
-    // k_onchip_solve
     const std::int32_t* fine_col;
     const double* fine_vd64;
     const double* rhs64;
@@ -71,10 +64,11 @@ struct OnchipArgs {
     int max_iterations, max_refinements;
 };
 
-// Device limits and launches, one translation unit per precision. R: fine rows per thread
-// of the solve kernel (1, 2, 4 or, in FP32, 7; 0: the cycle kernel).
+constexpr unsigned kOnchipThreads = 384;   // a block's at most
+
+// One translation unit per precision. R: fine rows per thread (1, 2, 4 or, in FP32, 7).
 template <typename T>
-unsigned onchip_shared_limit(int rows_per_thread);
+bool onchip_has(int rows_per_thread);
 // Whether the solve kernel keeps its fine rows in registers (else in shared memory).
 template <typename T>
 constexpr bool onchip_held(int rows_per_thread) { return sizeof(T) * rows_per_thread <= 16; }

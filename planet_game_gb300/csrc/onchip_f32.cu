@@ -3,8 +3,7 @@
 
 namespace psgb {
 
-template unsigned onchip_shared_limit<float>(int);
-template unsigned onchip_max_threads<float>(int);
+template bool onchip_has<float>(int);
 template int onchip_active_clusters<float>(int, unsigned, unsigned, std::size_t);
 template void onchip_launch<float>(const OnchipArgs<float>&, int, unsigned, std::size_t, cudaStream_t);
 

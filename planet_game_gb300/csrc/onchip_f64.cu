@@ -3,8 +3,7 @@
 
 namespace psgb {
 
-template unsigned onchip_shared_limit<double>(int);
-template unsigned onchip_max_threads<double>(int);
+template bool onchip_has<double>(int);
 template int onchip_active_clusters<double>(int, unsigned, unsigned, std::size_t);
 template void onchip_launch<double>(const OnchipArgs<double>&, int, unsigned, std::size_t, cudaStream_t);
 

@@ -338,7 +338,7 @@ __device__ int build_cycle(const Block& k, const OnchipArgs<T>& a, Phase* out) {
         }
         out[n++] = p;
     };
-    for (int l = a.first; l < a.coarsest; ++l) {
+    for (int l = 0; l < a.coarsest; ++l) {
         const OnchipLevel<T>& L = a.level[l];
         bool in_x = L.starts_in_x != 0;
         for (int s = 1; s < L.pre; ++s, in_x = !in_x) add(L.inner > 1 ? kBlockSweep : kSweep, l, in_x);
@@ -346,7 +346,7 @@ __device__ int build_cycle(const Block& k, const OnchipArgs<T>& a, Phase* out) {
         add(kRestrict, l, in_x);
     }
     add(kDense, a.coarsest, true);
-    for (int l = a.coarsest - 1; l >= a.first; --l) {
+    for (int l = a.coarsest - 1; l >= 0; --l) {
         const OnchipLevel<T>& L = a.level[l];
         bool in_x = (L.starts_in_x != 0) == (((L.pre - 1) & 1) == 0);   // where the sweeps down ended
         add(kProlong, l, in_x);
@@ -619,6 +619,12 @@ __device__ __forceinline__ void write_partials(const Block& k, std::uint32_t par
         scatter(part, static_cast<std::uint32_t>(rank), static_cast<std::uint32_t>(i) * stride + chunk0 + static_cast<std::uint32_t>(chunk), mine);
 }
 
+template <typename T>
+__device__ __forceinline__ int planet_of(const OnchipArgs<T>& a) {
+    const unsigned i = blockIdx.x / static_cast<unsigned>(a.cluster);
+    return static_cast<int>(a.list != nullptr ? a.list[i] : i);
+}
+
 // ---- the whole solve ------------------------------------------------------------------------------
 
 // Rows of the fine level a thread keeps in registers: matrix, addresses, aggregate.
@@ -854,13 +860,17 @@ struct Solve {
     }
 };
 
-template <typename T, int R, int MaxThreads>
-__global__ void __launch_bounds__(MaxThreads, 1) k_onchip_solve(const __grid_constant__ OnchipArgs<T> a) {
+// At most kOnchipThreads threads a block. Few threads with several rows each: the cluster
+// barrier is cheaper (0.19 us with 256 threads, 0.29 with 1024), and the whole solve, its rows'
+// matrix and addresses with it, stays in registers, where 1024 threads would spill to an L1 that
+// the shared memory leaves no room in.
+template <typename T, int R>
+__global__ void __launch_bounds__(kOnchipThreads, 1) k_onchip_solve(const __grid_constant__ OnchipArgs<T> a) {
     extern __shared__ __align__(16) unsigned char onchip_smem[];
     __shared__ Reduce red;
     const Block k = block_of(onchip_smem);
     Phase* const list = k.at<Phase>(a.o_list);
-    const int inst = static_cast<int>(a.list[blockIdx.x / static_cast<unsigned>(a.cluster)]);
+    const int inst = planet_of(a);
     if (a.active != nullptr && a.active[inst] == 0) {   // the whole cluster
         if (k.rank == 0 && k.tid == 0) {
             InstanceScalars& s = a.sc[inst];
@@ -966,62 +976,7 @@ __global__ void __launch_bounds__(MaxThreads, 1) k_onchip_solve(const __grid_con
     cluster_barrier();   // no block leaves while another may still read its shared memory
 }
 
-// ---- the coarse levels of one V-cycle -----------------------------------------------------------
-
-template <typename T>
-__global__ void __launch_bounds__(512, 1) k_onchip_cycle(const __grid_constant__ OnchipArgs<T> a) {
-    extern __shared__ __align__(16) unsigned char onchip_smem[];
-    __shared__ int phases;
-    const Block k = block_of(onchip_smem);
-    Phase* const list = k.at<Phase>(a.o_list);
-    const int inst = static_cast<int>(a.list[blockIdx.x / static_cast<unsigned>(a.cluster)]);
-    const auto first_row = [&](int l) { return a.tile_range[(l * a.instances + inst) * 2] * static_cast<std::uint32_t>(kTile); };
-    if (k.tid == 0) phases = build_cycle(k, a, list);
-    // The hierarchy was assembled before the solve's first launch: it loads while the launch
-    // before this one drains (through L2; nothing of it is written during the solve).
-    for (int l = a.first; l < a.coarsest; ++l) {
-        load_coarse(k, a.level[l], a.level[l + 1], first_row(l), first_row(l + 1));
-        load_members(k, a.level[l], a.level[l + 1], first_row(l), first_row(l + 1));
-    }
-    load_dense(k, a, inst);
-    pdl_begin();
-    if (!ph::gate_open(a.sc, inst, a.gate)) return;   // the whole cluster
-    const OnchipLevel<T>& F = a.level[a.first];
-    const int rows = own_rows(F.n, F.span, k.rank);
-    const std::size_t g0 = first_row(a.first) + std::size_t(k.rank) * F.span;
-    const T* start = F.starts_in_x ? F.gx : F.gy;
-    for (int i = k.tid; i < rows; i += k.threads) {
-        k.at<T>(F.o_b)[i] = __ldcg(&F.gb[g0 + i]);
-        k.at<T>(F.starts_in_x ? F.o_x : F.o_y)[i] = __ldcg(&start[g0 + i]);
-    }
-    cluster_barrier();
-    Ahead<T> ahead;
-    Phase p = list[0];
-    load_ahead(k, p, p.kind, k.tid, ahead);
-#pragma unroll 1
-    for (int i = 0;;) {
-        coarse_phase(k, p, p.kind, ahead, a.cluster, a.omega);
-        cluster_arrive();
-        if (++i < phases) {
-            p = list[i];
-            load_ahead(k, p, p.kind, k.tid, ahead);
-        }
-        cluster_wait();
-        if (i >= phases) break;
-    }
-    for (int i = k.tid; i < rows; i += k.threads) F.gx[g0 + i] = k.at<T>(F.o_x)[i];
-    cluster_barrier();
-}
-
 // ---- host side of one precision -------------------------------------------------------------------
-
-// Threads a block of the kernel may have. Few threads with several rows each: the cluster
-// barrier is cheaper (0.19 us with 256 threads, 0.29 with 1024), and the whole solve, its rows'
-// matrix and addresses with it, stays in registers, where 1024 threads would spill to an L1 that
-// the shared memory leaves no room in.
-constexpr unsigned max_threads(int rows_per_thread) {
-    return rows_per_thread == 0 ? 512u : 384u;
-}
 
 template <typename T>
 using KernelOf = void (*)(OnchipArgs<T>);
@@ -1029,12 +984,11 @@ using KernelOf = void (*)(OnchipArgs<T>);
 template <typename T>
 KernelOf<T> kernel_of(int rows_per_thread) {
     switch (rows_per_thread) {
-        case 0: return k_onchip_cycle<T>;
-        case 1: return k_onchip_solve<T, 1, max_threads(1)>;
-        case 2: return k_onchip_solve<T, 2, max_threads(2)>;
-        case 4: return k_onchip_solve<T, 4, max_threads(4)>;
+        case 1: return k_onchip_solve<T, 1>;
+        case 2: return k_onchip_solve<T, 2>;
+        case 4: return k_onchip_solve<T, 4>;
         case 7:
-            if constexpr (sizeof(T) == 4) return k_onchip_solve<T, 7, max_threads(7)>;
+            if constexpr (sizeof(T) == 4) return k_onchip_solve<T, 7>;
             return nullptr;
         default: return nullptr;
     }
@@ -1073,39 +1027,33 @@ unsigned shared_limit(int rows_per_thread) {
 }
 
 struct Config {
-    cudaLaunchAttribute attr[2];
+    cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg{};
-    Config(unsigned cluster, unsigned blocks, unsigned threads, std::size_t bytes, cudaStream_t st, bool early) {
+    Config(unsigned cluster, unsigned blocks, unsigned threads, std::size_t bytes, cudaStream_t st) {
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = cluster;
         attr[0].val.clusterDim.y = 1;
         attr[0].val.clusterDim.z = 1;
-        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[1].val.programmaticStreamSerializationAllowed = 1;
         cfg.gridDim = dim3(blocks);
         cfg.blockDim = dim3(threads);
         cfg.dynamicSmemBytes = bytes;
         cfg.stream = st;
         cfg.attrs = attr;
-        cfg.numAttrs = early ? 2 : 1;
+        cfg.numAttrs = 1;
     }
 };
 
 }  // namespace oc
 
 template <typename T>
-unsigned onchip_shared_limit(int rows_per_thread) {
-    return oc::shared_limit<T>(rows_per_thread);
-}
-template <typename T>
-unsigned onchip_max_threads(int rows_per_thread) {
-    return oc::kernel_of<T>(rows_per_thread) == nullptr ? 0u : oc::max_threads(rows_per_thread);
+bool onchip_has(int rows_per_thread) {
+    return oc::kernel_of<T>(rows_per_thread) != nullptr;
 }
 
 template <typename T>
 int onchip_active_clusters(int rows_per_thread, unsigned cluster, unsigned threads, std::size_t shared_bytes) {
     if (shared_bytes > oc::shared_limit<T>(rows_per_thread)) return 0;
-    oc::Config c(cluster, cluster, threads, shared_bytes, nullptr, false);
+    oc::Config c(cluster, cluster, threads, shared_bytes, nullptr);
     int clusters = 0;
     if (cudaOccupancyMaxActiveClusters(&clusters, oc::kernel_of<T>(rows_per_thread), &c.cfg) != cudaSuccess) {
         cudaGetLastError();
@@ -1119,8 +1067,8 @@ void onchip_launch(const OnchipArgs<T>& args, int rows_per_thread, unsigned thre
                    cudaStream_t st) {
     if (shared_bytes > oc::shared_limit<T>(rows_per_thread)) throw std::logic_error("on-chip solve: the planet does not fit");
     const unsigned cluster = static_cast<unsigned>(args.cluster);
-    oc::Config c(cluster, args.planets * cluster, threads, shared_bytes, st, rows_per_thread == 0);
-    PSGB_LAUNCH(rows_per_thread == 0 ? kFamSmoothCoarse : kFamPersistent, st, {
+    oc::Config c(cluster, args.planets * cluster, threads, shared_bytes, st);
+    PSGB_LAUNCH(kFamPersistent, st, {
         const cudaError_t e = cudaLaunchKernelEx(&c.cfg, oc::kernel_of<T>(rows_per_thread), args);
         if (e != cudaSuccess) throw std::runtime_error(std::string("on-chip solve launch: ") + cudaGetErrorString(e));
     });

@@ -14,8 +14,7 @@ namespace psgb {
 // The planets of one shape (the same rows on every level) and their launch.
 struct OnchipClass {
     std::vector<std::uint32_t> planets;   // indices in the batch
-    std::uint32_t* list = nullptr;        // the same on the device
-    std::size_t list_capacity = 0;
+    std::uint32_t* list = nullptr;        // the same on the device (null: every planet of the batch)
     unsigned cluster = 0, threads = 0;    // 0: not solved on chip
     int rows_per_thread = 0;
     int phases = 0;                       // of a V-cycle
