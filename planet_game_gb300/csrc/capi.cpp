@@ -771,14 +771,17 @@ int psgb_transport_step_multi(psgb_planet* h, const psgb_step_params* params, co
         int worst = PSGB_OK;
         for (uint32_t j = 0; j < count; ++j) {
             psgb::mr::take(P0, static_cast<int>(j), sp.xr, b.xr, st);
-            psgb::launch_step_finish(v, b.xr, in[j], in[psgb::mr::kRhs + j], b.hout, b.tnew, b.partial, b.sums, st);
+            psgb::launch_step_finish(v, b.xr, in[j], in[psgb::mr::kRhs + j], b.hout, b.tnew, b.partial, sp.sums + 8 * j, st);
             copy_out(t_new_K[j], b.tnew, n * 8, memory, st);
             if (transport_W_m2 != nullptr && transport_W_m2[j] != nullptr) {
                 copy_out(transport_W_m2[j], b.hout, n * 8, memory, st);
             }
-            double sums[8];
-            PSGB_CUDA(cudaMemcpyAsync(sums, b.sums, sizeof(sums), cudaMemcpyDeviceToHost, st));
-            PSGB_CUDA(cudaStreamSynchronize(st));
+        }
+        std::vector<double> all_sums(8 * std::size_t(count));
+        PSGB_CUDA(cudaMemcpyAsync(all_sums.data(), sp.sums, all_sums.size() * sizeof(double), cudaMemcpyDeviceToHost, st));
+        PSGB_CUDA(cudaStreamSynchronize(st));
+        for (uint32_t j = 0; j < count; ++j) {
+            const double* sums = &all_sums[8 * std::size_t(j)];
             psgb_step_report local;
             fill_report(sp.host[j], &local.solve);
             local.sum_W = sums[0];

@@ -185,6 +185,7 @@ void prepare(Batch& b, Space& s, const SolveOptions& opt) {
         s.bb = zeroed<double>(s.store, P0 * kRhs);
         s.part = zeroed<double>(s.store, 2 * std::size_t(b.levels[0].tiles) * kRhs);
         s.sc = zeroed<InstanceScalars>(s.store, kRhs);
+        s.sums = zeroed<double>(s.store, 8 * std::size_t(kRhs));
         s.pointers = s.store.alloc<const double*>(2 * kRhs);
         PSGB_CUDA(cudaMallocHost(&s.pinned, kRhs * sizeof(InstanceScalars)));
         s.host.assign(kRhs, InstanceScalars{});

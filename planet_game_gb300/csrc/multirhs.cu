@@ -114,6 +114,56 @@ __device__ __forceinline__ void stage_rows(const LevelView<T>& L, int tile, Tile
     __syncthreads();
 }
 
+// The V-cycle's sweeps, residuals and prolongations reduce nothing, so their rows may go to any
+// block. On levels of few tiles a block takes a 32-row slice of a tile (block = tile * 8 +
+// slice), a warp four of its rows, all their loads in flight at once: one block per tile with a
+// warp per 32 rows in turn left them to a few blocks (level 7, 32 right-hand sides, FP32: a sweep
+// on 41 tiles 18.3 us, on 3 tiles 17.7; a prolongation 37.8 and 35.3; sliced 7.0, 6.1, 7.5 and
+// 6.6). On levels that fill the GPU with tiles the tile's rows stay together, its neighbours'
+// lines shared through L1 (641 tiles: 22.5 us a sweep, sliced 30.0).
+constexpr unsigned kSlicedTiles = 2 * 152;
+constexpr int kSlice = 32;                     // rows of a block
+constexpr int kSlices = kTile / kSlice;        // blocks of a tile
+constexpr int kSliceRows = kSlice / 8;         // rows of a warp
+
+template <typename T, int W, bool Diag, bool Inv>
+struct SliceRows {
+    int col[W][kSlice];
+    T val[W + (Diag ? 1 : 0)][kSlice];
+    T inv[Inv ? kSlice : 1];
+};
+
+// The slice's matrix rows, staged with coalesced loads (thread t: slot t / 32, row t % 32).
+template <typename T, int W, bool Diag, bool Inv>
+__device__ __forceinline__ void stage_slice(const LevelView<T>& L, int first, SliceRows<T, W, Diag, Inv>& m) {
+    const std::uint32_t P = L.rows;
+    const int r = threadIdx.x & (kSlice - 1);
+#pragma unroll
+    for (int j = threadIdx.x / kSlice; j < W; j += kTile / kSlice) {
+        m.col[j][r] = L.col[j * P + first + r];
+        m.val[j][r] = L.vd[j * P + first + r];
+    }
+    // (the slots past W fall to the threads that the loop above leaves free first)
+    if constexpr (Diag) {
+        if (threadIdx.x / kSlice == kTile / kSlice - 1) m.val[W][r] = L.vd[W * P + first + r];
+    }
+    if constexpr (Inv) {
+        if (threadIdx.x / kSlice == kTile / kSlice - 2) m.inv[r] = L.inv[first + r];
+    }
+    __syncthreads();
+}
+
+struct Slice {
+    int tile, local0, rows;   // the warp's first row within the tile; the tile's valid rows
+    bool on;                  // the slice has rows to smooth
+};
+__device__ __forceinline__ Slice slice_of(const std::uint32_t* meta) {
+    const int tile = static_cast<int>(blockIdx.x) / kSlices, part = static_cast<int>(blockIdx.x) % kSlices;
+    const TileInfo ti = tile_info(meta, tile);
+    return Slice{tile, part * kSlice + static_cast<int>(threadIdx.x >> 5) * kSliceRows, ti.rows,
+                 ti.sweep && part * kSlice < ti.rows};
+}
+
 // ---- V-cycle ----------------------------------------------------------------------------
 
 template <typename T>
@@ -166,6 +216,39 @@ __global__ void k_smooth(LevelView<T> L, const T* __restrict__ b, const T* __res
             const int local = local_row(warp, g, i);
             if (local < ti.rows) y[at(tile * kTile + local, lane)] = out[i];
         }
+    }
+}
+
+template <typename T, int W>
+__global__ void k_smooth_slices(LevelView<T> L, const T* __restrict__ b, const T* __restrict__ x, T* __restrict__ y, T omega,
+                         const InstanceScalars* sc, int gate) {
+    pdl_begin();
+    const int lane = threadIdx.x & 31;
+    const Slice sl = slice_of(L.tile_meta);
+    if (!sl.on) return;
+    const int first = sl.tile * kTile, slice0 = sl.local0 & ~(kSlice - 1);
+    __shared__ SliceRows<T, W, false, true> m;
+    stage_slice(L, first + slice0, m);
+    if (blockIdx.x % kSlices == 0)
+        count(L.bytes, static_cast<unsigned long long>(sl.rows) * (4ull * W + sizeof(T) * (W + 1ull) + 3ull * kRhs * sizeof(T)));
+    if (!ph::gate_open(sc, lane, gate)) return;
+    T out[kSliceRows];
+#pragma unroll
+    for (int i = 0; i < kSliceRows; ++i) {
+        const int local = sl.local0 - slice0 + i, row = first + sl.local0 + i;
+        T s = b[at(row, lane)];
+#pragma unroll
+        for (int j = 0; j < W; ++j) s -= m.val[j][local] * x[at(m.col[j][local], lane)];
+        if (omega == T(1)) {
+            out[i] = m.inv[local] * s;
+        } else {
+            const T xo = x[at(row, lane)];
+            out[i] = xo + omega * (m.inv[local] * s - xo);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kSliceRows; ++i) {
+        if (sl.local0 + i < sl.rows) y[at(first + sl.local0 + i, lane)] = out[i];
     }
 }
 
@@ -285,36 +368,63 @@ __global__ void k_residual(LevelView<T> L, const T* __restrict__ b, const T* __r
     }
 }
 
-// b_c = sum of the members' residuals in ascending order; x_c = omega b_c / diag.
+template <typename T, int W>
+__global__ void k_residual_slices(LevelView<T> L, const T* __restrict__ b, const T* __restrict__ x, T* __restrict__ r,
+                           const InstanceScalars* sc, int gate) {
+    pdl_begin();
+    const int lane = threadIdx.x & 31;
+    const Slice sl = slice_of(L.tile_meta);
+    if (!sl.on) return;
+    const int first = sl.tile * kTile, slice0 = sl.local0 & ~(kSlice - 1);
+    __shared__ SliceRows<T, W, true, false> m;
+    stage_slice(L, first + slice0, m);
+    if (blockIdx.x % kSlices == 0)
+        count(L.bytes, static_cast<unsigned long long>(sl.rows) * (4ull * W + sizeof(T) * (W + 1ull) + 3ull * kRhs * sizeof(T)));
+    if (!ph::gate_open(sc, lane, gate)) return;
+    T out[kSliceRows];
+#pragma unroll
+    for (int i = 0; i < kSliceRows; ++i) {
+        const int local = sl.local0 - slice0 + i, row = first + sl.local0 + i;
+        T s = b[at(row, lane)] - m.val[W][local] * x[at(row, lane)];
+#pragma unroll
+        for (int j = 0; j < W; ++j) s -= m.val[j][local] * x[at(m.col[j][local], lane)];
+        out[i] = s;
+    }
+#pragma unroll
+    for (int i = 0; i < kSliceRows; ++i) {
+        if (sl.local0 + i < sl.rows) r[at(first + sl.local0 + i, lane)] = out[i];
+    }
+}
+
+// b_c = sum of the members' residuals in ascending order; x_c = omega b_c / diag. One warp a
+// coarse row (block = tile * 32 + eight rows), sixteen members' lines in flight: 32 rows a warp in
+// turn took 89 us on level 7's 10,242 coarse rows and 71 on its 42.
 template <typename T>
 __global__ void k_restrict_zero(LevelView<T> C, const std::uint32_t* __restrict__ moff,
                                 const std::uint32_t* __restrict__ member, const T* __restrict__ r,
                                 T* __restrict__ bc, T* __restrict__ xc, T omega, const InstanceScalars* sc, int gate) {
     pdl_begin();
-    const int tile = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    constexpr int kBlocks = kTile / 8;
+    const int tile = static_cast<int>(blockIdx.x) / kBlocks, lane = threadIdx.x & 31;
+    const int local = static_cast<int>(blockIdx.x) % kBlocks * 8 + static_cast<int>(threadIdx.x >> 5);
     const TileInfo ti = tile_info(C.tile_meta, tile);
-    if (ti.rows == 0 || !ph::gate_open(sc, lane, gate)) return;
-    unsigned long long moved = 0;
-    for (int k = 0; k < 32; ++k) {
-        const int local = warp * 32 + k;
-        if (local >= ti.rows) break;
-        const int row = tile * kTile + local;
-        const std::uint32_t k0 = moff[row], k1 = moff[row + 1];
-        T s = T(0);
-        for (std::uint32_t m = k0; m < k1; m += 8) {
-            T v[8];
+    if (local >= ti.rows || !ph::gate_open(sc, lane, gate)) return;
+    const int row = tile * kTile + local;
+    const std::uint32_t k0 = moff[row], k1 = moff[row + 1];
+    T s = T(0);
+    for (std::uint32_t m = k0; m < k1; m += 16) {
+        T v[16];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = (m + u < k1) ? r[at(static_cast<int>(member[m + u]), lane)] : T(0);
+        for (int u = 0; u < 16; ++u) v[u] = (m + u < k1) ? r[at(static_cast<int>(member[m + u]), lane)] : T(0);
 #pragma unroll
-            for (int u = 0; u < 8; ++u) {
-                if (m + u < k1) s += v[u];
-            }
+        for (int u = 0; u < 16; ++u) {
+            if (m + u < k1) s += v[u];
         }
-        bc[at(row, lane)] = s;
-        if (ti.sweep) xc[at(row, lane)] = omega * C.inv[row] * s;
-        moved += 4ull + (k1 - k0) * (4ull + kRhs * sizeof(T)) + sizeof(T) + 2ull * kRhs * sizeof(T);
     }
-    if (C.bytes != nullptr && lane == 0 && moved != 0) atomicAdd(C.bytes, moved);
+    bc[at(row, lane)] = s;
+    if (ti.sweep) xc[at(row, lane)] = omega * C.inv[row] * s;
+    if (C.bytes != nullptr && lane == 0)
+        atomicAdd(C.bytes, 4ull + (k1 - k0) * (4ull + kRhs * sizeof(T)) + sizeof(T) + 2ull * kRhs * sizeof(T));
 }
 
 // With x' = x + e[agg]: y = x' + omega (D^-1 (b - O x') - x').
@@ -356,6 +466,43 @@ __global__ void k_prolong_smooth(LevelView<T> L, const std::int32_t* __restrict_
     }
 }
 
+template <typename T, int W>
+__global__ void k_prolong_smooth_slices(LevelView<T> L, const std::int32_t* __restrict__ agg, const T* __restrict__ e,
+                                 const T* __restrict__ b, const T* __restrict__ x, T* __restrict__ y, T omega,
+                                 const InstanceScalars* sc, int gate) {
+    pdl_begin();
+    const int lane = threadIdx.x & 31;
+    const Slice sl = slice_of(L.tile_meta);
+    if (!sl.on) return;
+    const int first = sl.tile * kTile, slice0 = sl.local0 & ~(kSlice - 1);
+    __shared__ SliceRows<T, W, false, true> m;
+    stage_slice(L, first + slice0, m);
+    if (blockIdx.x % kSlices == 0)
+        count(L.bytes, static_cast<unsigned long long>(sl.rows) * (4ull * W + sizeof(T) * (W + 1ull) + 4ull + 3ull * kRhs * sizeof(T)));
+    if (!ph::gate_open(sc, lane, gate)) return;
+    T out[kSliceRows];
+#pragma unroll
+    for (int i = 0; i < kSliceRows; ++i) {
+        const int local = sl.local0 - slice0 + i, row = first + sl.local0 + i;
+        T s = b[at(row, lane)];
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            const int c = m.col[j][local];
+            s -= m.val[j][local] * (x[at(c, lane)] + ph::prod(L.correction, e[at(agg[c], lane)]));
+        }
+        if (omega == T(1)) {
+            out[i] = m.inv[local] * s;
+        } else {
+            const T xo = x[at(row, lane)] + ph::prod(L.correction, e[at(agg[row], lane)]);
+            out[i] = xo + omega * (m.inv[local] * s - xo);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < kSliceRows; ++i) {
+        if (sl.local0 + i < sl.rows) y[at(first + sl.local0 + i, lane)] = out[i];
+    }
+}
+
 template <typename T>
 __global__ void k_prolong(LevelView<T> L, const std::int32_t* __restrict__ agg, const T* __restrict__ xc, T* x,
                           const InstanceScalars* sc, int gate) {
@@ -373,6 +520,29 @@ __global__ void k_prolong(LevelView<T> L, const std::int32_t* __restrict__ agg, 
     }
 }
 
+template <typename T>
+__global__ void k_prolong_slices(LevelView<T> L, const std::int32_t* __restrict__ agg, const T* __restrict__ xc, T* x,
+                          const InstanceScalars* sc, int gate) {
+    pdl_begin();
+    const int lane = threadIdx.x & 31;
+    const Slice sl = slice_of(L.tile_meta);
+    if (!sl.on) return;
+    if (blockIdx.x % kSlices == 0)
+        count(L.bytes, static_cast<unsigned long long>(sl.rows) * (4ull + 2ull * kRhs * sizeof(T)));
+    if (!ph::gate_open(sc, lane, gate)) return;
+    T xo[kSliceRows], c[kSliceRows];
+#pragma unroll
+    for (int i = 0; i < kSliceRows; ++i) {
+        const int row = sl.tile * kTile + sl.local0 + i;
+        xo[i] = x[at(row, lane)];
+        c[i] = xc[at(agg[row], lane)];
+    }
+#pragma unroll
+    for (int i = 0; i < kSliceRows; ++i) {
+        if (sl.local0 + i < sl.rows) x[at(sl.tile * kTile + sl.local0 + i, lane)] = xo[i] + ph::prod(L.correction, c[i]);
+    }
+}
+
 // Coarsest level: x = A^-1 b, row i in warp i of the grid, lane = right-hand side. The
 // single solve's warp sums a[k] b[k] over k = l, l + 32, ... in lane l, then the butterfly
 // over l; here each lane forms those 32 sums itself, in the butterfly's pairing.
@@ -386,17 +556,22 @@ __global__ void k_dense(int n, const T* __restrict__ inv, const T* __restrict__ 
     if (bytes != nullptr && lane == 0) atomicAdd(bytes, static_cast<unsigned long long>(n) * sizeof(T) + kRhs * sizeof(T));
     if (!ph::gate_open(sc, lane, gate)) return;
     const T* a = inv + static_cast<std::size_t>(i) * n;
-    T run[8];
+    // the 32 sums side by side, 32 entries of b in flight (one sum after the other took 21 us)
+    T acc[32], run[8];
+#pragma unroll
+    for (int l = 0; l < 32; ++l) acc[l] = T(0);
+    for (int k = 0; k < n; k += 32) {
+        T v[32];
+#pragma unroll
+        for (int l = 0; l < 32; ++l) v[l] = k + l < n ? b[at(k + l, lane)] : T(0);
+#pragma unroll
+        for (int l = 0; l < 32; ++l) {
+            if (k + l < n) acc[l] += a[k + l] * v[l];
+        }
+    }
 #pragma unroll
     for (int g = 0; g < 8; ++g) {
-        T v[4];
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            const int l = g + 8 * u;
-            T s = T(0);
-            for (int k = l; k < n; k += 32) s += a[k] * b[at(k, lane)];
-            v[u] = s;
-        }
+        const T v[4] = {acc[g], acc[g + 8], acc[g + 16], acc[g + 24]};
         run[g] = run_value(v);
     }
     x[at(i, lane)] = butterfly(run);
@@ -749,6 +924,16 @@ __global__ void k_take(std::uint32_t P, int j, const double* __restrict__ x, dou
         default: throw std::logic_error("unsupported ELL width");              \
     }
 
+// Whether a level's sweeps run in slices, and their blocks.
+template <typename T>
+bool sliced(const LevelView<T>& L) {
+    return L.tiles < kSlicedTiles;
+}
+template <typename T>
+unsigned blocks_of(const LevelView<T>& L) {
+    return sliced(L) ? L.tiles * kSlices : L.tiles;
+}
+
 template <int K>
 void finish(const Ctx& ctx, int tiles, int family, cudaStream_t st, ph::FinishParams p = {}) {
     PSGB_LAUNCH(family, st, launch_pdl(k_finish<K>, kRhs, kTile, st, ctx, tiles, p));
@@ -783,35 +968,36 @@ void Launch<T>::smooth(const LevelView<T>& L, const T* b, const T* x, T* y, T om
         }));
         return;
     }
-    PSGB_LAUNCH(fam, st, PSGB_MR_WIDTHS(L.width, launch_pdl(k_smooth<T, W>, L.tiles, kTile, st, counted(L, fam), b, x, y,
-                                                            omega, sc, gate)));
+    PSGB_LAUNCH(fam, st, PSGB_MR_WIDTHS(L.width, launch_pdl(sliced(L) ? k_smooth_slices<T, W> : k_smooth<T, W>, blocks_of(L),
+                                                            kTile, st, counted(L, fam), b, x, y, omega, sc, gate)));
 }
 template <typename T>
 void Launch<T>::residual(const LevelView<T>& L, const T* b, const T* x, T* r, const InstanceScalars* sc, int gate,
                          cudaStream_t st) {
     const int fam = L.level == 0 ? kFamResidual : kFamResidualCoarse;
-    PSGB_LAUNCH(fam, st, PSGB_MR_WIDTHS(L.width, launch_pdl(k_residual<T, W>, L.tiles, kTile, st, counted(L, fam), b, x,
-                                                            r, sc, gate)));
+    PSGB_LAUNCH(fam, st, PSGB_MR_WIDTHS(L.width, launch_pdl(sliced(L) ? k_residual_slices<T, W> : k_residual<T, W>,
+                                                            blocks_of(L), kTile, st, counted(L, fam), b, x, r, sc, gate)));
 }
 template <typename T>
 void Launch<T>::restrict_zero(const LevelView<T>& C, const std::uint32_t* moff, const std::uint32_t* member, const T* r,
                               T* bc, T* xc, T omega, const InstanceScalars* sc, int gate, cudaStream_t st) {
     const int fam = C.level <= 1 ? kFamRestrict : kFamRestrictCoarse;
-    PSGB_LAUNCH(fam, st, launch_pdl(k_restrict_zero<T>, C.tiles, kTile, st, counted(C, fam), moff, member, r, bc, xc,
+    PSGB_LAUNCH(fam, st, launch_pdl(k_restrict_zero<T>, C.tiles * (kTile / 8), kTile, st, counted(C, fam), moff, member, r, bc, xc,
                                     omega, sc, gate));
 }
 template <typename T>
 void Launch<T>::prolong_smooth(const LevelView<T>& L, const std::int32_t* agg, const T* e, const T* b, const T* x,
                                T* y, T omega, const InstanceScalars* sc, int gate, cudaStream_t st) {
     const int fam = L.level == 0 ? kFamSmooth : kFamSmoothCoarse;
-    PSGB_LAUNCH(fam, st, PSGB_MR_WIDTHS(L.width, launch_pdl(k_prolong_smooth<T, W>, L.tiles, kTile, st, counted(L, fam),
-                                                            agg, e, b, x, y, omega, sc, gate)));
+    PSGB_LAUNCH(fam, st, PSGB_MR_WIDTHS(L.width, launch_pdl(sliced(L) ? k_prolong_smooth_slices<T, W> : k_prolong_smooth<T, W>,
+                                                            blocks_of(L), kTile, st, counted(L, fam), agg, e, b, x, y, omega,
+                                                            sc, gate)));
 }
 template <typename T>
 void Launch<T>::prolong(const LevelView<T>& L, const std::int32_t* agg, const T* xc, T* x, const InstanceScalars* sc,
                         int gate, cudaStream_t st) {
     const int fam = L.level == 0 ? kFamProlong : kFamProlongCoarse;
-    PSGB_LAUNCH(fam, st, launch_pdl(k_prolong<T>, L.tiles, kTile, st, counted(L, fam), agg, xc, x, sc, gate));
+    PSGB_LAUNCH(fam, st, launch_pdl(sliced(L) ? k_prolong_slices<T> : k_prolong<T>, blocks_of(L), kTile, st, counted(L, fam), agg, xc, x, sc, gate));
 }
 template <typename T>
 void Launch<T>::dense(int n, const T* inv, const T* b, T* x, const InstanceScalars* sc, int gate, cudaStream_t st) {

@@ -79,6 +79,7 @@ struct Space {
     double* rr = nullptr;     // residual, FP64
     double* bb = nullptr;     // right-hand sides, FP64
     double* part = nullptr;   // [2][tiles of the fine level][kRhs]
+    double* sums = nullptr;   // [32][8] the steps' energy sums
     InstanceScalars* sc = nullptr;
     InstanceScalars* pinned = nullptr;
     const double** pointers = nullptr;   // device [2][kRhs]: the sub-steps' T0 and S
