@@ -114,8 +114,10 @@ void launch_galerkin(std::uint32_t lists, const std::uint32_t* offset, const std
                      const double* fine_vd, double* coarse_vd, cudaStream_t stream);
 void launch_finalize_level(std::uint32_t rows, std::uint32_t width, double* vd64, float* vd32,
                            double* inv64, float* inv32, cudaStream_t stream);
-void launch_dense_invert(const DenseView& dense, int level, const LevelView<double>& lv,
-                         double* work, double* inv64, float* inv32, cudaStream_t stream);
+// dense_invert.cu: the inverses of the `planets` planets whose coarsest level is `level`, the
+// largest of `max_rows` rows.
+void launch_dense_invert(const DenseView& dense, int level, const LevelView<double>& lv, std::uint32_t max_rows,
+                         std::uint32_t planets, double* inv64, float* inv32, cudaStream_t stream);
 
 template <typename T>
 void launch_smooth_zero(const LevelView<T>& lv, const T* b, T* x, T omega, const InstanceScalars* sc,

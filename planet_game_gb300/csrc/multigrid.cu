@@ -110,56 +110,6 @@ __global__ void k_finalize_level(std::uint32_t P, std::uint32_t W, double* __res
     inv32[row] = static_cast<float>(inv);
 }
 
-// Dense inverse of every planet's coarsest level (symmetric positive definite):
-// assemble from the ELL values, then in-place Gauss-Jordan without pivoting. One CTA
-// per planet; the matrix lives in global memory (<= 400 x 400 doubles).
-__global__ void __launch_bounds__(1024) k_dense_invert(DenseView dense, int level, LevelView<double> lv,
-                                                       double* __restrict__ work,
-                                                       double* __restrict__ inv64,
-                                                       float* __restrict__ inv32) {
-    pdl_begin();
-    const int inst = blockIdx.x;
-    if (dense.level[inst] != level) return;
-    const int n = static_cast<int>(dense.size[inst]);
-    const std::int64_t base = dense.row_base[inst];
-    double* a = work + dense.offset[inst];
-    const std::uint32_t P = lv.rows, W = lv.width;
-    for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) a[idx] = 0.0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        const std::int64_t row = base + i;
-        a[i * n + i] = lv.vd[W * P + row];
-        for (std::uint32_t j = 0; j < W; ++j) {
-            const std::int64_t c = lv.col[j * P + row];
-            if (c == row) continue;
-            a[i * n + (c - base)] += lv.vd[j * P + row];
-        }
-    }
-    __syncthreads();
-    __shared__ double f[400];
-    __shared__ double pivot_inv;
-    for (int k = 0; k < n; ++k) {
-        if (threadIdx.x == 0) pivot_inv = 1.0 / a[k * n + k];
-        __syncthreads();
-        for (int j = threadIdx.x; j < n; j += blockDim.x) {
-            a[k * n + j] = (j == k ? 1.0 : a[k * n + j]) * pivot_inv;
-        }
-        for (int i = threadIdx.x; i < n; i += blockDim.x) f[i] = a[i * n + k];
-        __syncthreads();
-        for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
-            const int i = idx / n, j = idx - i * n;
-            if (i == k) continue;
-            const double aij = (j == k) ? 0.0 : a[idx];
-            a[idx] = aij - f[i] * a[k * n + j];
-        }
-        __syncthreads();
-    }
-    for (int idx = threadIdx.x; idx < n * n; idx += blockDim.x) {
-        inv64[dense.offset[inst] + idx] = a[idx];
-        inv32[dense.offset[inst] + idx] = static_cast<float>(a[idx]);
-    }
-}
-
 // ---- V-cycle pieces: one 256-thread block per tile (the shared phases of phases.cuh) ----
 
 template <typename T, int R>
@@ -378,11 +328,6 @@ void launch_galerkin(std::uint32_t lists, const std::uint32_t* offset, const std
 void launch_finalize_level(std::uint32_t rows, std::uint32_t width, double* vd64, float* vd32,
                            double* inv64, float* inv32, cudaStream_t stream) {
     PSGB_LAUNCH(kFamSetup, stream, launch_pdl(k_finalize_level, (rows + 255) / 256, 256, stream, rows, width, vd64, vd32, inv64, inv32));
-}
-
-void launch_dense_invert(const DenseView& dense, int level, const LevelView<double>& lv,
-                         double* work, double* inv64, float* inv32, cudaStream_t stream) {
-    PSGB_LAUNCH(kFamSetup, stream, launch_pdl(k_dense_invert, dense.instances, 1024, stream, dense, level, lv, work, inv64, inv32));
 }
 
 template <typename T>

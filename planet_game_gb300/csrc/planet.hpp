@@ -178,7 +178,6 @@ struct DenseCoarse {
     int2* d_blocks = nullptr;
     double* inv64 = nullptr;           // concatenated row-major inverses
     float* inv32 = nullptr;
-    double* work = nullptr;
     std::int32_t* d_level = nullptr;
     std::uint64_t* d_offset = nullptr;
     std::uint32_t* d_size = nullptr;

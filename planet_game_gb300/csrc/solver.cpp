@@ -401,7 +401,6 @@ std::unique_ptr<Batch> build_batch(const std::vector<Planet*>& planets, void* ar
     D.d_blocks = b.store.upload(blocks);
     D.inv64 = b.store.alloc<double>(total);
     D.inv32 = b.store.alloc<float>(total);
-    D.work = b.store.alloc<double>(total);
     D.d_level = b.store.upload(D.level);
     D.d_offset = b.store.upload(D.offset);
     D.d_size = b.store.upload(D.size);
@@ -695,11 +694,14 @@ void prepare_levels(Batch& b, cudaStream_t st) {
     }
     const DenseView dv = dense_view(b);
     for (std::size_t l = 0; l < b.levels.size(); ++l) {
-        bool any = false;
-        for (auto c : b.dense.level) any = any || (c == static_cast<int>(l));
-        if (!any) continue;
-        launch_dense_invert(dv, static_cast<int>(l), view64(b, l), b.dense.work, b.dense.inv64,
-                            b.dense.inv32, st);
+        std::uint32_t planets = 0, rows = 0;
+        for (std::uint32_t i = 0; i < b.instances; ++i) {
+            if (b.dense.level[i] != static_cast<int>(l)) continue;
+            ++planets;
+            rows = std::max(rows, b.dense.size[i]);
+        }
+        if (planets == 0) continue;
+        launch_dense_invert(dv, static_cast<int>(l), view64(b, l), rows, planets, b.dense.inv64, b.dense.inv32, st);
     }
     PSGB_CUDA(cudaGetLastError());
     b.matrix_ready = true;
