@@ -122,18 +122,26 @@ IluPattern ilu_pattern(const std::vector<std::uint32_t>& offset, const std::vect
     if (fits) {
         for (int part = 0; part < 2; ++part) {
             LevelSchedule& s = part == 0 ? p.lower : p.upper;
+            const auto begin = [&](std::uint32_t i) { return part == 0 ? p.start[i] : p.diagonal[i] + 1; };
+            const auto end = [&](std::uint32_t i) { return part == 0 ? p.diagonal[i] : p.start[i + 1]; };
+            // rows of one level by their number of couplings, so that a warp's rows have as many
+            // (any order within a level gives the same factor and solve)
+            for (std::size_t lv = 0; lv + 1 < s.level_start.size(); ++lv) {
+                std::stable_sort(s.order.begin() + s.level_start[lv], s.order.begin() + s.level_start[lv + 1],
+                                 [&](std::uint32_t a, std::uint32_t b) { return end(a) - begin(a) > end(b) - begin(b); });
+            }
             s.rec_row.resize(p.rows);
             s.rec_count.resize(p.rows);
             s.rec_col.assign(std::size_t(p.rows) * kIluRecord, 0);
             s.rec_q.assign(std::size_t(p.rows) * kIluRecord, 0);
             for (std::uint32_t b = 0; b < p.blocks; ++b) {
+                s.deepest = std::max(s.deepest, s.block_level[b + 1] - s.block_level[b]);
                 for (std::uint32_t lv = s.block_level[b]; lv < s.block_level[b + 1]; ++lv) {
                     s.widest = std::max(s.widest, s.level_start[lv + 1] - s.level_start[lv]);
                     for (std::uint32_t idx = s.level_start[lv]; idx < s.level_start[lv + 1]; ++idx) {
                         const std::uint32_t i = s.order[idx];
                         const std::uint32_t first = block_start[b];
-                        const std::uint32_t q0 = part == 0 ? p.start[i] : p.diagonal[i] + 1;
-                        const std::uint32_t q1 = part == 0 ? p.diagonal[i] : p.start[i + 1];
+                        const std::uint32_t q0 = begin(i), q1 = end(i);
                         s.rec_row[idx] = static_cast<std::uint16_t>(i - first);
                         s.rec_count[idx] = static_cast<std::uint8_t>(q1 - q0);
                         for (std::uint32_t q = q0; q < q1; ++q) {

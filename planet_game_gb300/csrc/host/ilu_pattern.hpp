@@ -29,6 +29,7 @@ struct LevelSchedule {
     std::vector<std::uint16_t> rec_col;       // [rows][kIluRecord]
     std::vector<std::uint32_t> rec_q;         // [rows][kIluRecord]
     std::uint32_t widest = 0;                 // most rows in one level
+    std::uint32_t deepest = 0;                // most levels in one block
 };
 
 constexpr int kIluRecord = 8;

@@ -91,7 +91,8 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_factor(IluView v) {
 }
 
 // x <- (LU)^-1 x (incomplete_lu.cpp:137-152): forward, then backward, level by level.
-__global__ void __launch_bounds__(kIluThreads) k_ilu_solve(IluView v, double* __restrict__ x) {
+__global__ void __launch_bounds__(kIluThreads) k_ilu_solve(IluView v, double* __restrict__ x, const int* skip) {
+    if (skip != nullptr && *skip != 0) return;
     const std::uint32_t b = blockIdx.x;
     for (std::uint32_t lv = v.lo_block[b]; lv < v.lo_block[b + 1]; ++lv) {
         for (std::uint32_t idx = v.lo_level[lv] + threadIdx.x; idx < v.lo_level[lv + 1]; idx += kIluThreads) {
@@ -115,17 +116,29 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_solve(IluView v, double* __
 
 // The triangular solves with the block's x in shared memory and per-level records (the
 // row, its couplings' block-local columns and their factor values packed next to them):
-// a thread owns one row of a level, loads the next level's record before the current
-// level's barrier, so a level costs a barrier and shared-memory reads rather than a chain
-// of dependent global loads. Same terms in the same order as k_ilu_solve: same bits.
+// a thread owns one row of a level and loads the next level's record before the current
+// level computes. Same terms in the same order as k_ilu_solve: same bits.
+//
+//
+// A level is a few dozen to a few hundred rows of up to eight products and differences each, and
+// on the way back a division. An SM starts an FP64 instruction of a warp every 19 cycles, the
+// same warp's next one after 66, and one lane costs what 32 do: the levels are bound by these
+// instructions. So a warp's rows have the same number of couplings and the terms that none of them
+// has are not issued (as selections, every row paid for eight); the division by the diagonal is
+// five operations on its stored reciprocal (Markstein, IBM J. Res. Dev. 34, 1990: with r = RN(1/d)
+// and a quotient q within one unit in the last place, RN(q + r (s - d q)) is RN(s/d); one such step
+// from q = RN(s r) gives that quotient, the next rounds it); and a level's records are
+// loaded, one value a plane, while the level before computes. A pair of SMs a block, half of each level's rows on either, was slower: its barrier and
+// the store to the partner take 400 to 900 cycles a level, as much as the halves save.
+// Ten layers on 10,242 nodes, 41 blocks of 2,560 rows in 23 levels each way: 51 us a
+// solve, 86 before.
 struct IluRecords {
-    const std::uint16_t* row;
-    const std::uint8_t* count;
-    const std::uint16_t* col;      // [rows][8]
+    const std::uint32_t* head;     // the row and, from bit 16, its couplings
+    const uint4* cols;             // eight 16-bit columns
+    double* val;                   // [8][rows]: packed after each factorisation
+    double2* diag;                 // upper: the diagonal and its reciprocal (0: divide)
     const std::uint32_t* q;        // [rows][8]: value positions
-    double* val;                   // [rows][8]: packed values
     const std::uint32_t* dq;       // upper: the row's diagonal position
-    double* dval;                  // upper: the diagonal value
     const std::uint32_t* block;    // [blocks + 1] levels
     const std::uint32_t* level;    // [levels + 1]
 };
@@ -133,80 +146,125 @@ struct IluRecords {
 struct IluShared {
     IluRecords lo, up;
     const std::uint32_t* block_start;   // [blocks + 1] rows
+    std::uint32_t rows;
 };
 
 __global__ void k_ilu_pack(std::uint32_t rows, IluShared s, const double* __restrict__ value) {
     const std::uint32_t idx = blockIdx.x * kThreads + threadIdx.x;
     if (idx >= rows) return;
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        s.lo.val[idx * 8 + k] = k < s.lo.count[idx] ? value[s.lo.q[idx * 8 + k]] : 0.0;
-        s.up.val[idx * 8 + k] = k < s.up.count[idx] ? value[s.up.q[idx * 8 + k]] : 0.0;
+    for (std::uint32_t k = 0; k < 8; ++k) {
+        s.lo.val[k * rows + idx] = k < s.lo.head[idx] >> 16 ? value[s.lo.q[idx * 8 + k]] : 0.0;
+        s.up.val[k * rows + idx] = k < s.up.head[idx] >> 16 ? value[s.up.q[idx * 8 + k]] : 0.0;
     }
-    s.up.dval[idx] = value[s.up.dq[idx]];
+    const double d = value[s.up.dq[idx]];
+    s.up.diag[idx] = make_double2(d, fabs(d) > 0x1p-100 && fabs(d) < 0x1p100 ? 1.0 / d : 0.0);
 }
 
+// A row's record as it is loaded; nothing here is looked at before its level.
 struct Rec {
-    int row, count;
-    std::uint16_t col[8];
+    std::uint32_t head;
+    uint4 cols;
     double val[8];
-    double diag;
+    double2 diag;
 };
 
-__device__ __forceinline__ Rec load_rec(const IluRecords& r, std::uint32_t lv, bool upper) {
-    Rec x;
-    x.row = -1;
-    x.count = 0;
-    x.diag = 1.0;
-    const std::uint32_t idx = r.level[lv] + threadIdx.x;
-    if (idx < r.level[lv + 1]) {
-        x.row = r.row[idx];
-        x.count = r.count[idx];
-        const uint4 c = *reinterpret_cast<const uint4*>(r.col + std::size_t(idx) * 8);
-        const std::uint16_t* cc = reinterpret_cast<const std::uint16_t*>(&c);
+// The row's differences, for a warp whose rows have at most N couplings; a lane with fewer takes
+// off +0, which changes nothing.
+template <int N>
+__device__ __forceinline__ double subtract_terms(const Rec& c, const double* xs, double sum) {
+    const std::uint32_t count = c.head >> 16;
+    double p[N];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) x.col[k] = cc[k];
-        const double2* v = reinterpret_cast<const double2*>(r.val + std::size_t(idx) * 8);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            const double2 d = v[k];
-            x.val[2 * k] = d.x;
-            x.val[2 * k + 1] = d.y;
-        }
-        if (upper) x.diag = r.dval[idx];
+    for (std::uint32_t k = 0; k < N; ++k) {
+        const std::uint32_t w = k < 2 ? c.cols.x : k < 4 ? c.cols.y : k < 6 ? c.cols.z : c.cols.w;
+        p[k] = k < count ? xs[k & 1 ? w >> 16 : w & 0xffffu] : 0.0;
     }
-    return x;
+#pragma unroll
+    for (int k = 0; k < N; ++k) p[k] = c.val[k] * p[k];
+#pragma unroll
+    for (int k = 0; k < N; ++k) sum -= p[k];
+    return sum;
+}
+
+// s / d, correctly rounded, from r = RN(1/d) of a diagonal of ordinary size (0: divide). The
+// magnitude is looked at in whole numbers: a comparison of doubles takes the FP64 unit as long as
+// a product.
+__device__ __forceinline__ double quotient(double s, double d, double r) {
+    const std::uint32_t high = static_cast<std::uint32_t>(__double2hiint(s)) & 0x7fffffffu;
+    constexpr std::uint32_t low = (1023u - 800u) << 20, span = 1600u << 20;   // 2^-800 <= |s| < 2^800
+    if (__double2hiint(r) != 0 && high - low < span) {
+        double q = s * r;
+        q = __fma_rn(__fma_rn(-d, q, s), r, q);
+        return __fma_rn(__fma_rn(-d, q, s), r, q);
+    }
+    if (__double2hiint(r) != 0 && (high | static_cast<std::uint32_t>(__double2loint(s))) == 0u) return s * r;
+    return s / d;
 }
 
 constexpr unsigned kIluSharedThreads = 512;   // the widest level the shared-memory solve takes
 
-__global__ void __launch_bounds__(kIluSharedThreads, 1) k_ilu_solve_shared(IluShared s, double* __restrict__ x) {
-    extern __shared__ double xs[];
+// out <- (LU)^-1 in, the same vector or another; a thread block a block of the matrix, a thread a
+// row of each level. `skip`: a device word that, where set, makes the solve needless (null: always
+// run). `deepest`: most levels of one triangle.
+__global__ void __launch_bounds__(kIluSharedThreads, 1) k_ilu_solve_shared(IluShared s, const double* in, double* out,
+                                                                          const int* skip, std::uint32_t deepest) {
+    if (skip != nullptr && *skip != 0) return;
+    extern __shared__ double ilu_smem[];
+    double* xs = ilu_smem;
     const std::uint32_t b = blockIdx.x;
     const std::uint32_t first = s.block_start[b], n = s.block_start[b + 1] - first;
-    for (std::uint32_t r = threadIdx.x; r < n; r += blockDim.x) xs[r] = x[first + r];
+    std::uint32_t* starts = reinterpret_cast<std::uint32_t*>(xs + n);   // level starts of both triangles
+    const std::uint32_t lo0 = s.lo.block[b], lo_levels = s.lo.block[b + 1] - lo0;
+    const std::uint32_t up0 = s.up.block[b], levels = lo_levels + s.up.block[b + 1] - up0;
+    for (std::uint32_t l = threadIdx.x; l <= lo_levels; l += blockDim.x) starts[l] = s.lo.level[lo0 + l];
+    for (std::uint32_t l = threadIdx.x; l <= levels - lo_levels; l += blockDim.x) starts[deepest + 1 + l] = s.up.level[up0 + l];
+    for (std::uint32_t r = threadIdx.x; r < n; r += blockDim.x) xs[r] = in[first + r];
     __syncthreads();
-    for (int part = 0; part < 2; ++part) {
-        const bool upper = part == 1;
+    // levels 0 .. lo_levels there, the others back
+    const auto level = [&](std::uint32_t lv) {
+        return starts + (lv < lo_levels ? lv : deepest + 1 + lv - lo_levels);
+    };
+    const auto load = [&](std::uint32_t lv) {
+        const bool upper = lv >= lo_levels;
         const IluRecords& R = upper ? s.up : s.lo;
-        const std::uint32_t lv0 = R.block[b], lv1 = R.block[b + 1];
-        const Rec none{-1, 0, {}, {}, 1.0};
-        // the next level's record loads while this level computes and meets
-        Rec cur = lv0 < lv1 ? load_rec(R, lv0, upper) : none;
-        for (std::uint32_t lv = lv0; lv < lv1; ++lv) {
-            const Rec next = lv + 1 < lv1 ? load_rec(R, lv + 1, upper) : none;
-            if (cur.row >= 0) {
-                double sum = xs[cur.row];
+        const std::uint32_t* st = level(lv);
+        const std::uint32_t idx = lv < levels ? st[0] + threadIdx.x : 0u;
+        Rec c{0xffffu, make_uint4(0u, 0u, 0u, 0u), {}, make_double2(1.0, 0.0)};
+        if (lv < levels && idx < st[1]) {
+            c.head = R.head[idx];
+            c.cols = R.cols[idx];
 #pragma unroll
-                for (int k = 0; k < 8; ++k)
-                    if (k < cur.count) sum -= cur.val[k] * xs[cur.col[k]];
-                xs[cur.row] = upper ? sum / cur.diag : sum;
-            }
-            __syncthreads();
-            cur = next;
+            for (std::uint32_t k = 0; k < 8; ++k) c.val[k] = R.val[std::size_t(k) * s.rows + idx];
+            if (upper) c.diag = R.diag[idx];
         }
+        return c;
+    };
+    Rec c = load(0);
+    for (std::uint32_t lv = 0; lv < levels; ++lv) {
+        const Rec next = load(lv + 1);
+        const std::uint32_t row = c.head & 0xffffu;
+        const bool on = row != 0xffffu;   // at most 4096 rows
+        double sum = on ? xs[row] : 0.0;
+        switch (__shfl_sync(0xffffffffu, c.head >> 16, 0)) {   // the most of the warp: a level's rows are in falling order
+            case 0: break;
+            case 1: sum = subtract_terms<1>(c, xs, sum); break;
+            case 2: sum = subtract_terms<2>(c, xs, sum); break;
+            case 3: sum = subtract_terms<3>(c, xs, sum); break;
+            case 4: sum = subtract_terms<4>(c, xs, sum); break;
+            case 5: sum = subtract_terms<5>(c, xs, sum); break;
+            case 6: sum = subtract_terms<6>(c, xs, sum); break;
+            case 7: sum = subtract_terms<7>(c, xs, sum); break;
+            default: sum = subtract_terms<8>(c, xs, sum); break;
+        }
+        if (on) {
+            if (lv >= lo_levels) sum = quotient(sum, c.diag.x, c.diag.y);
+            xs[row] = sum;
+        }
+        __syncthreads();
+        c = next;
     }
-    for (std::uint32_t r = threadIdx.x; r < n; r += blockDim.x) x[first + r] = xs[r];
+    for (std::uint32_t r = threadIdx.x; r < n; r += blockDim.x) out[first + r] = xs[r];
 }
 
 }  // namespace
@@ -236,18 +294,20 @@ class DeviceIlu {
         if (!p.lower.rec_row.empty() && widest <= kIluSharedThreads) {
             auto records = [&](const LevelSchedule& sch, bool upper) {
                 IluRecords r{};
-                r.row = store_.upload(sch.rec_row);
-                r.count = store_.upload(sch.rec_count);
-                r.col = store_.upload(sch.rec_col);
-                r.q = store_.upload(sch.rec_q);
+                std::vector<std::uint32_t> head(p.rows);
+                for (std::uint32_t idx = 0; idx < p.rows; ++idx)
+                    head[idx] = sch.rec_row[idx] | static_cast<std::uint32_t>(sch.rec_count[idx]) << 16;
+                r.head = store_.upload(head);
+                r.cols = reinterpret_cast<const uint4*>(store_.upload(sch.rec_col));
                 r.val = store_.alloc<double>(sch.rec_q.size());
+                r.q = store_.upload(sch.rec_q);
                 r.block = upper ? v_.up_block : v_.lo_block;
                 r.level = upper ? v_.up_level : v_.lo_level;
                 if (upper) {
                     std::vector<std::uint32_t> dq(p.rows);
                     for (std::uint32_t idx = 0; idx < p.rows; ++idx) dq[idx] = p.diagonal[sch.order[idx]];
                     r.dq = store_.upload(dq);
-                    r.dval = store_.alloc<double>(p.rows);
+                    r.diag = store_.alloc<double2>(p.rows);
                 }
                 return r;
             };
@@ -263,8 +323,11 @@ class DeviceIlu {
                 most = std::max(most, count);
             }
             shared_.block_start = store_.upload(starts);
-            shared_threads_ = std::max(32u, (widest + 31) / 32 * 32);
-            shared_bytes_ = std::max<std::size_t>(8, std::size_t(most) * sizeof(double));
+            deepest_ = std::max(p.lower.deepest, p.upper.deepest);
+            shared_threads_ = std::max(1u, (widest + 31) / 32) * 32;
+            shared_.rows = p.rows;
+            // at most 4096 rows and so as many levels: 64 KB
+            shared_bytes_ = std::size_t(most) * sizeof(double) + 2 * (std::size_t(deepest_) + 1) * sizeof(std::uint32_t);
             use_shared_ = shared_bytes_ <= 48 * 1024 ||
                           cudaFuncSetAttribute(k_ilu_solve_shared, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                static_cast<int>(shared_bytes_)) == cudaSuccess;
@@ -290,11 +353,14 @@ class DeviceIlu {
         if (flag != 0) throw Breakdown("incomplete LU: zero pivot");
     }
 
-    void solve(double* x, cudaStream_t st) const {
+    // out <- (LU)^-1 in (the same vector, or another). `skip`: a device word; the solve is left
+    // out where it is set.
+    void solve(const double* in, double* out, cudaStream_t st, const int* skip = nullptr) const {
         if (use_shared_) {
-            k_ilu_solve_shared<<<blocks_, shared_threads_, shared_bytes_, st>>>(shared_, x);
+            k_ilu_solve_shared<<<blocks_, shared_threads_, shared_bytes_, st>>>(shared_, in, out, skip, deepest_);
         } else {
-            k_ilu_solve<<<blocks_, kIluThreads, 0, st>>>(v_, x);
+            if (in != out) PSGB_CUDA(cudaMemcpyAsync(out, in, std::size_t(rows_) * 8, cudaMemcpyDeviceToDevice, st));
+            k_ilu_solve<<<blocks_, kIluThreads, 0, st>>>(v_, out, skip);
         }
         PSGB_CHECK_LAUNCH();
     }
@@ -307,6 +373,7 @@ class DeviceIlu {
     std::uint32_t rows_, blocks_;
     IluShared shared_{};
     bool use_shared_ = false;
+    std::uint32_t deepest_ = 0;
     unsigned shared_threads_ = 0;
     std::size_t shared_bytes_ = 0;
 };
@@ -349,22 +416,6 @@ __device__ double tree_max(double v, double* sh) {
 
 constexpr int kQ = 4;   // quantities per block partial
 
-// Block partials of up to two dots: u1.v1, u2.v2 (u2 null: one).
-__global__ void __launch_bounds__(kThreads) k_dots(std::uint32_t n, const double* __restrict__ u1,
-                                                   const double* __restrict__ v1, const double* __restrict__ u2,
-                                                   const double* __restrict__ v2, double* __restrict__ partial) {
-    __shared__ double sh[kThreads];
-    const std::uint32_t i = blockIdx.x * kThreads + threadIdx.x;
-    const double a = i < n ? u1[i] * v1[i] : 0.0;
-    const double s1 = tree_sum(a, sh);
-    double s2 = 0.0;
-    if (u2 != nullptr) s2 = tree_sum(i < n ? u2[i] * v2[i] : 0.0, sh);
-    if (threadIdx.x == 0) {
-        partial[blockIdx.x * kQ + 0] = s1;
-        partial[blockIdx.x * kQ + 1] = s2;
-    }
-}
-
 // One block: the partials of `quantities` values in fixed order; bit q of max_mask: a max.
 __global__ void __launch_bounds__(kThreads) k_finish(unsigned blocks, int quantities, unsigned max_mask,
                                                      const double* __restrict__ partial, double* __restrict__ out) {
@@ -381,34 +432,138 @@ __global__ void __launch_bounds__(kThreads) k_finish(unsigned blocks, int quanti
     }
 }
 
-__global__ void k_copy(std::uint32_t n, const double* __restrict__ a, double* __restrict__ b) {
-    const std::uint32_t i = blockIdx.x * kThreads + threadIdx.x;
-    if (i < n) b[i] = a[i];
+// BiCGSTAB's scalars on the device: each step of the iteration is decided where its sums are
+// finished, by the last block of the kernel that forms them, so that the host only looks in from
+// time to time and the GPU never waits for it. 102,420 rows: an iteration's vectors, products and
+// sums 55 us beside its two solves; with kernels for the sums alone, read back and decided by the
+// host, 130 us.
+struct BicgState {
+    int done;         // nothing runs any more
+    int half;         // converged at s: x += alpha p_hat closes the solve
+    int skip_second;  // done or half
+    int iteration, max_iterations;
+    unsigned arrived;   // blocks of the kernel under way
+    double rho, alpha, omega, beta, b_norm, tolerance;
+};
+
+enum BicgSum : int { kSumStart, kSumV, kSumS, kSumT, kSumX };
+
+__device__ void bicg_step(BicgState& s, int kind, double a, double b) {
+    const auto next = [&](double rho_next) {   // the head of an iteration
+        if (s.iteration >= s.max_iterations || rho_next == 0.0 || s.omega == 0.0) {
+            s.done = 1;
+        } else {
+            s.beta = rho_next / s.rho * (s.alpha / s.omega);
+            s.rho = rho_next;
+        }
+    };
+    if (kind == kSumStart) {          // b . b (and shadow . r, the same sum)
+        s.b_norm = sqrt(a);
+        s.rho = s.alpha = s.omega = 1.0;
+        if (!(s.b_norm > 0.0)) s.done = 1;
+        else next(a);
+    } else if (kind == kSumV) {       // shadow . v
+        if (a == 0.0) s.done = 1;
+        else s.alpha = s.rho / a;
+    } else if (kind == kSumS) {       // s . s
+        ++s.iteration;
+        if (sqrt(a) <= s.tolerance * s.b_norm) s.half = 1;
+    } else if (kind == kSumT) {       // t . t, t . s
+        s.omega = a > 0.0 ? b / a : 0.0;
+    } else if (s.half != 0 || sqrt(a) <= s.tolerance * s.b_norm) {   // r . r, shadow . r
+        s.done = 1;
+    } else {
+        next(b);
+    }
+    s.skip_second = s.done | s.half;
 }
-__global__ void k_bicg_p(std::uint32_t n, const double* __restrict__ r, double* __restrict__ p,
-                         const double* __restrict__ v, double beta, double omega) {
-    const std::uint32_t i = blockIdx.x * kThreads + threadIdx.x;
-    if (i < n) p[i] = r[i] + beta * (p[i] - omega * v[i]);
-}
-__global__ void k_bicg_s(std::uint32_t n, const double* __restrict__ r, const double* __restrict__ v, double alpha,
-                         double* __restrict__ s) {
-    const std::uint32_t i = blockIdx.x * kThreads + threadIdx.x;
-    if (i < n) s[i] = r[i] - alpha * v[i];
-}
-__global__ void k_bicg_x1(std::uint32_t n, double* __restrict__ x, const double* __restrict__ p_hat, double alpha) {
-    const std::uint32_t i = blockIdx.x * kThreads + threadIdx.x;
-    if (i < n) x[i] += alpha * p_hat[i];
-}
-__global__ void k_bicg_xr(std::uint32_t n, double* __restrict__ x, double* __restrict__ r,
-                          const double* __restrict__ p_hat, const double* __restrict__ s_hat,
-                          const double* __restrict__ s, const double* __restrict__ t, double alpha, double omega) {
-    const std::uint32_t i = blockIdx.x * kThreads + threadIdx.x;
-    if (i < n) {
-        x[i] += alpha * p_hat[i] + omega * s_hat[i];
-        r[i] = s[i] - omega * t[i];
+
+// A block's sums of one or two quantities; the last block to arrive sums all blocks' in fixed order
+// (k_finish's) and takes the step. Every block has read the state by then.
+__device__ __forceinline__ void sum_and_step(int kind, double a, double b, double* sh, double* partial, BicgState* state) {
+    __shared__ bool last;
+    const bool two = kind == kSumT || kind == kSumX;
+    const double s1 = tree_sum(a, sh);
+    const double s2 = two ? tree_sum(b, sh) : 0.0;
+    if (threadIdx.x == 0) {
+        partial[blockIdx.x * kQ + 0] = s1;
+        partial[blockIdx.x * kQ + 1] = s2;
+        __threadfence();
+        last = atomicAdd(&state->arrived, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double v[2] = {0.0, 0.0};
+    for (unsigned k = threadIdx.x; k < gridDim.x; k += kThreads) {
+        v[0] = v[0] + __ldcg(&partial[k * kQ]);
+        if (two) v[1] = v[1] + __ldcg(&partial[k * kQ + 1]);
+    }
+    const double sum = tree_sum(v[0], sh);
+    const double other = two ? tree_sum(v[1], sh) : 0.0;
+    if (threadIdx.x == 0) {
+        state->arrived = 0;
+        bicg_step(*state, kind, sum, other);
     }
 }
 
+__global__ void __launch_bounds__(kThreads) k_bicg_start(std::uint32_t n, const double* __restrict__ b,
+                                                         double* __restrict__ x, double* __restrict__ r,
+                                                         double* __restrict__ shadow, double* __restrict__ p,
+                                                         double* __restrict__ v, BicgState* state, double* partial) {
+    __shared__ double sh[kThreads];
+    const std::uint32_t i = blockIdx.x * kThreads + threadIdx.x;
+    const double bv = i < n ? b[i] : 0.0;
+    if (i < n) {
+        x[i] = 0.0;
+        r[i] = bv;
+        shadow[i] = bv;
+        p[i] = 0.0;
+        v[i] = 0.0;
+    }
+    sum_and_step(kSumStart, i < n ? bv * bv : 0.0, 0.0, sh, partial, state);
+}
+__global__ void k_bicg_p(std::uint32_t n, const double* __restrict__ r, double* __restrict__ p,
+                         const double* __restrict__ v, const BicgState* state) {
+    if (state->done != 0) return;
+    const double beta = state->beta, omega = state->omega;
+    const std::uint32_t i = blockIdx.x * kThreads + threadIdx.x;
+    if (i < n) p[i] = r[i] + beta * (p[i] - omega * v[i]);
+}
+__global__ void __launch_bounds__(kThreads) k_bicg_s(std::uint32_t n, const double* __restrict__ r,
+                                                     const double* __restrict__ v, double* __restrict__ s,
+                                                     BicgState* state, double* partial) {
+    __shared__ double sh[kThreads];
+    if (state->done != 0) return;
+    const double alpha = state->alpha;
+    const std::uint32_t i = blockIdx.x * kThreads + threadIdx.x;
+    double sv = 0.0;
+    if (i < n) {
+        sv = r[i] - alpha * v[i];
+        s[i] = sv;
+    }
+    sum_and_step(kSumS, i < n ? sv * sv : 0.0, 0.0, sh, partial, state);
+}
+__global__ void __launch_bounds__(kThreads) k_bicg_x(std::uint32_t n, double* __restrict__ x, double* __restrict__ r,
+                                                     const double* __restrict__ p_hat, const double* __restrict__ s_hat,
+                                                     const double* __restrict__ s, const double* __restrict__ t,
+                                                     const double* __restrict__ shadow, BicgState* state,
+                                                     double* partial) {
+    __shared__ double sh[kThreads];
+    if (state->done != 0) return;
+    const double alpha = state->alpha, omega = state->omega;
+    const std::uint32_t i = blockIdx.x * kThreads + threadIdx.x;
+    double rv = 0.0, dv = 0.0;
+    if (state->half != 0) {
+        if (i < n) x[i] += alpha * p_hat[i];
+    } else if (i < n) {
+        x[i] += alpha * p_hat[i] + omega * s_hat[i];
+        rv = s[i] - omega * t[i];
+        r[i] = rv;
+        dv = shadow[i] * rv;
+    }
+    sum_and_step(kSumX, i < n ? rv * rv : 0.0, dv, sh, partial, state);
+}
 
 // y = diag x + off x (the reference's apply) on an ELL copy of the off-diagonals (slot-major,
 // coalesced): slot j of row r is CSR entry offset[r] + j, so the terms add in the same
@@ -427,32 +582,63 @@ __global__ void k_csr_to_ell(Ell e, const std::uint32_t* __restrict__ offset, co
     for (std::uint32_t j = 0; j < e.width; ++j) val[std::size_t(j) * e.rows + r] = j < deg ? off[first + j] : 0.0;
 }
 
-__global__ void k_ell_apply(Ell e, const double* __restrict__ val, const double* __restrict__ diag,
-                            const double* __restrict__ x, double* __restrict__ y) {
-    const std::uint32_t r = blockIdx.x * kThreads + threadIdx.x;
-    if (r >= e.rows) return;
+// A row's product, its loads in flight together where the row is at most eight wide.
+__device__ __forceinline__ double ell_row(const Ell& e, const double* __restrict__ val, const double* __restrict__ diag,
+                                          const double* __restrict__ x, std::uint32_t r) {
     const std::uint32_t deg = e.degree[r];
     double sum = diag[r] * x[r];
+    if (e.width <= 8) {
+        double v[8], g[8];
+#pragma unroll
+        for (std::uint32_t j = 0; j < 8; ++j) {
+            const std::size_t at = std::size_t(j < e.width ? j : 0u) * e.rows + r;
+            v[j] = val[at];
+            g[j] = x[e.col[at]];
+        }
+#pragma unroll
+        for (std::uint32_t j = 0; j < 8; ++j) {
+            if (j < deg) sum += v[j] * g[j];
+        }
+        return sum;
+    }
     for (std::uint32_t j = 0; j < e.width; ++j) {
         if (j < deg) sum += val[std::size_t(j) * e.rows + r] * x[e.col[std::size_t(j) * e.rows + r]];
     }
-    y[r] = sum;
+    return sum;
+}
+
+__global__ void k_ell_apply(Ell e, const double* __restrict__ val, const double* __restrict__ diag,
+                            const double* __restrict__ x, double* __restrict__ y) {
+    const std::uint32_t r = blockIdx.x * kThreads + threadIdx.x;
+    if (r < e.rows) y[r] = ell_row(e, val, diag, x, r);
+}
+
+// v = A p_hat and shadow . v; or t = A s_hat, t . t and t . s (`second`).
+__global__ void __launch_bounds__(kThreads) k_bicg_apply(Ell e, const double* __restrict__ val, const double* __restrict__ diag,
+                                                         const double* __restrict__ x, double* __restrict__ y,
+                                                         const double* __restrict__ u, bool second, BicgState* state,
+                                                         double* partial) {
+    __shared__ double sh[kThreads];
+    if (second ? state->skip_second != 0 : state->done != 0) return;
+    const std::uint32_t r = blockIdx.x * kThreads + threadIdx.x;
+    double yv = 0.0, uv = 0.0;
+    if (r < e.rows) {
+        yv = ell_row(e, val, diag, x, r);
+        y[r] = yv;
+        uv = u[r];
+    }
+    const bool on = r < e.rows;
+    const double yy = yv * yv, yu = yv * uv;
+    sum_and_step(second ? kSumT : kSumV, on ? (second ? yy : yu) : 0.0, on && second ? yu : 0.0, sh, partial, state);
 }
 
 // Device scratch and the scalars read back for the host's decisions.
 class Scalars {
   public:
-    Scalars(DeviceStore& store, std::size_t n) : blocks_(blocks_of(n)), n_(n) {
+    Scalars(DeviceStore& store, std::size_t n) : blocks_(blocks_of(n)) {
         partial_ = store.alloc<double>(std::size_t(blocks_) * kQ);
         out_ = store.alloc<double>(kQ);
         host_.reset(kQ);
-    }
-    // u1.v1 (and u2.v2)
-    std::pair<double, double> dots(const double* u1, const double* v1, const double* u2, const double* v2,
-                                   cudaStream_t st) {
-        k_dots<<<blocks_, kThreads, 0, st>>>(static_cast<std::uint32_t>(n_), u1, v1, u2, v2, partial_);
-        PSGB_CHECK_LAUNCH();
-        return read(u2 != nullptr ? 2 : 1, 0u, st);
     }
     double* partial() { return partial_; }
     unsigned blocks() const { return blocks_; }
@@ -467,69 +653,84 @@ class Scalars {
 
   private:
     unsigned blocks_;
-    std::size_t n_;
     double* partial_;
     double* out_;
     PinnedDoubles host_;
 };
 
-using Op = std::function<void(const double*, double*)>;
+// M^-1 x; `skip` a device word that, where set, makes it needless.
+using Precondition = std::function<void(const double*, double*, const int* skip)>;
 
-// BiCGSTAB's vectors, allocated once per solve.
+// BiCGSTAB's vectors, device state and the host's copies of it, kept with the caller's workspace.
 struct BicgWork {
     double *r, *shadow, *p, *v, *p_hat, *s, *s_hat, *t;
+    BicgState* state;
+    BicgState* host = nullptr;          // [2], pinned
+    cudaEvent_t seen[2] = {nullptr, nullptr};
     BicgWork(DeviceStore& store, std::size_t n)
         : r(store.alloc<double>(n)), shadow(store.alloc<double>(n)), p(store.alloc<double>(n)),
           v(store.alloc<double>(n)), p_hat(store.alloc<double>(n)), s(store.alloc<double>(n)),
-          s_hat(store.alloc<double>(n)), t(store.alloc<double>(n)) {}
+          s_hat(store.alloc<double>(n)), t(store.alloc<double>(n)), state(store.alloc<BicgState>(1)) {
+        PSGB_CUDA(cudaMallocHost(reinterpret_cast<void**>(&host), 2 * sizeof(BicgState)));
+        for (cudaEvent_t& e : seen) PSGB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
+    BicgWork(const BicgWork&) = delete;
+    BicgWork& operator=(const BicgWork&) = delete;
+    ~BicgWork() {
+        for (cudaEvent_t e : seen)
+            if (e != nullptr) cudaEventDestroy(e);
+        if (host != nullptr) cudaFreeHost(host);
+    }
 };
 
-// Right-preconditioned BiCGSTAB (heat_transport.cpp:823-897): x <- A^-1 b from x = 0.
-int bicgstab(std::size_t n, const Op& apply, const Op& precondition, const double* b, double* x, double tolerance,
-             int max_iterations, const BicgWork& work, Scalars& sc, cudaStream_t st) {
-    const std::uint32_t un = static_cast<std::uint32_t>(n);
+// Right-preconditioned BiCGSTAB (heat_transport.cpp:823-897): x <- A^-1 b from x = 0, A on its
+// ELL copy. `ahead`: the host queues one iteration more than it has seen the state of; what is
+// queued past the end finds `done` set and returns at once. A preconditioner that cannot be left
+// out on the device (a V-cycle of many launches) is not queued ahead: the host reads the state
+// before each one.
+int bicgstab(const Ell& ell, const double* val, const double* diag, const Precondition& precondition, bool ahead,
+             const double* b, double* x, double tolerance, int max_iterations, const BicgWork& w, Scalars& sc,
+             cudaStream_t st) {
+    const std::uint32_t n = ell.rows;
     const unsigned g = blocks_of(n);
-    double *r = work.r, *shadow = work.shadow, *p = work.p, *v = work.v, *p_hat = work.p_hat, *s = work.s,
-           *s_hat = work.s_hat, *t = work.t;
-    PSGB_CUDA(cudaMemsetAsync(x, 0, n * 8, st));
-    k_copy<<<g, kThreads, 0, st>>>(un, b, r);
-    k_copy<<<g, kThreads, 0, st>>>(un, b, shadow);
-    PSGB_CUDA(cudaMemsetAsync(p, 0, n * 8, st));
-    PSGB_CUDA(cudaMemsetAsync(v, 0, n * 8, st));
+    const int *done = &w.state->done, *skip_second = &w.state->skip_second;
+    BicgState begin{};
+    begin.max_iterations = max_iterations;
+    begin.tolerance = tolerance;
+    w.host[0] = begin;
+    PSGB_CUDA(cudaMemcpyAsync(w.state, &w.host[0], sizeof(BicgState), cudaMemcpyHostToDevice, st));
+    k_bicg_start<<<g, kThreads, 0, st>>>(n, b, x, w.r, w.shadow, w.p, w.v, w.state, sc.partial());
     PSGB_CHECK_LAUNCH();
-    const double b_norm = std::sqrt(sc.dots(b, b, nullptr, nullptr, st).first);
-    if (!(b_norm > 0.0)) return 0;
-    double rho = 1.0, alpha = 1.0, omega = 1.0;
-    int iteration = 0;
-    while (iteration < max_iterations) {
-        const double rho_next = sc.dots(shadow, r, nullptr, nullptr, st).first;
-        if (rho_next == 0.0 || omega == 0.0) break;
-        const double beta = rho_next / rho * (alpha / omega);
-        rho = rho_next;
-        k_bicg_p<<<g, kThreads, 0, st>>>(un, r, p, v, beta, omega);
-        PSGB_CHECK_LAUNCH();
-        precondition(p, p_hat);
-        apply(p_hat, v);
-        const double shadow_v = sc.dots(shadow, v, nullptr, nullptr, st).first;
-        if (shadow_v == 0.0) break;
-        alpha = rho / shadow_v;
-        k_bicg_s<<<g, kThreads, 0, st>>>(un, r, v, alpha, s);
-        PSGB_CHECK_LAUNCH();
-        ++iteration;
-        if (std::sqrt(sc.dots(s, s, nullptr, nullptr, st).first) <= tolerance * b_norm) {
-            k_bicg_x1<<<g, kThreads, 0, st>>>(un, x, p_hat, alpha);
-            PSGB_CHECK_LAUNCH();
-            break;
+    const auto read = [&]() -> const BicgState& {
+        PSGB_CUDA(cudaMemcpyAsync(&w.host[0], w.state, sizeof(BicgState), cudaMemcpyDeviceToHost, st));
+        PSGB_CUDA(cudaStreamSynchronize(st));
+        return w.host[0];
+    };
+    if (!ahead && read().done != 0) return 0;
+    for (int queued = 0; queued < std::max(1, max_iterations); ++queued) {
+        k_bicg_p<<<g, kThreads, 0, st>>>(n, w.r, w.p, w.v, w.state);
+        precondition(w.p, w.p_hat, done);
+        k_bicg_apply<<<g, kThreads, 0, st>>>(ell, val, diag, w.p_hat, w.v, w.shadow, false, w.state, sc.partial());
+        k_bicg_s<<<g, kThreads, 0, st>>>(n, w.r, w.v, w.s, w.state, sc.partial());
+        if (ahead || read().skip_second == 0) {
+            precondition(w.s, w.s_hat, skip_second);
+            k_bicg_apply<<<g, kThreads, 0, st>>>(ell, val, diag, w.s_hat, w.t, w.s, true, w.state, sc.partial());
         }
-        precondition(s, s_hat);
-        apply(s_hat, t);
-        const auto [t_t, t_s] = sc.dots(t, t, t, s, st);
-        omega = t_t > 0.0 ? t_s / t_t : 0.0;
-        k_bicg_xr<<<g, kThreads, 0, st>>>(un, x, r, p_hat, s_hat, s, t, alpha, omega);
+        k_bicg_x<<<g, kThreads, 0, st>>>(n, x, w.r, w.p_hat, w.s_hat, w.s, w.t, w.shadow, w.state, sc.partial());
+        if (!ahead) {
+            PSGB_CHECK_LAUNCH();
+            if (read().done != 0) break;
+            continue;
+        }
         PSGB_CHECK_LAUNCH();
-        if (std::sqrt(sc.dots(r, r, nullptr, nullptr, st).first) <= tolerance * b_norm) break;
+        const int slot = queued & 1;
+        PSGB_CUDA(cudaMemcpyAsync(&w.host[slot], w.state, sizeof(BicgState), cudaMemcpyDeviceToHost, st));
+        PSGB_CUDA(cudaEventRecord(w.seen[slot], st));
+        if (queued == 0) continue;
+        PSGB_CUDA(cudaEventSynchronize(w.seen[slot ^ 1]));
+        if (w.host[slot ^ 1].done != 0) return w.host[slot ^ 1].iteration;
     }
-    return iteration;
+    return ahead ? read().iteration : w.host[0].iteration;
 }
 
 // ---- advection-diffusion source ----------------------------------------------------
@@ -836,6 +1037,21 @@ __global__ void __launch_bounds__(kThreads) k_tracer_flux_form(GraphView g, Tran
 
 // ---- per-planet structures ------------------------------------------------------------
 
+// The tracer solve's vectors, kept with its stacked system: allocating and freeing two dozen of
+// them, and their pinned host copies, took 1.5 ms of every call.
+struct TracerWork {
+    DeviceStore store;
+    double *vertical, *divergence, *diagonal, *off, *rhs, *start, *applied, *residual, *delta, *solved, *off_ell;
+    Scalars scalars;
+    BicgWork bicg;
+    TracerWork(std::size_t rows, std::size_t nodes, std::size_t entries, std::size_t width)
+        : vertical(store.alloc<double>(rows)), divergence(store.alloc<double>(nodes)), diagonal(store.alloc<double>(rows)),
+          off(store.alloc<double>(entries)), rhs(store.alloc<double>(rows)), start(store.alloc<double>(rows)),
+          applied(store.alloc<double>(rows)), residual(store.alloc<double>(rows)), delta(store.alloc<double>(rows)),
+          solved(store.alloc<double>(rows)), off_ell(store.alloc<double>(width * rows)), scalars(store, rows),
+          bicg(store, rows) {}
+};
+
 struct NonsymContext {
     DeviceStore store;
     GraphView graph{};
@@ -849,6 +1065,7 @@ struct NonsymContext {
         Stacked view{};
         Ell ell{};
         std::unique_ptr<DeviceIlu> ilu;
+        std::unique_ptr<struct TracerWork> work;   // on the first solve
     };
     std::map<std::uint32_t, std::unique_ptr<StackedSystem>> stacked;
 };
@@ -1037,13 +1254,13 @@ int psgb_incomplete_lu_solve(psgb_incomplete_lu* h, double* x, int memory, void*
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         const std::size_t n = h->ilu->rows();
         if (memory == PSGB_MEMORY_DEVICE) {
-            h->ilu->solve(x, st);
+            h->ilu->solve(x, x, st);
             return PSGB_OK;
         }
         psgb::DeviceStore scratch;
         double* d = scratch.alloc<double>(n);
         PSGB_CUDA(cudaMemcpyAsync(d, x, n * 8, cudaMemcpyHostToDevice, st));
-        h->ilu->solve(d, st);
+        h->ilu->solve(d, d, st);
         PSGB_CUDA(cudaMemcpyAsync(x, d, n * 8, cudaMemcpyDeviceToHost, st));
         PSGB_CUDA(cudaStreamSynchronize(st));
         return PSGB_OK;
@@ -1104,16 +1321,12 @@ int psgb_solve_implicit_tracer(psgb_planet* planet, const psgb_advection_diffusi
         const double* c0 = psgb::input(w, tracer, std::size_t(L) * g.nodes, memory, st);
         const std::size_t rows = S.view.rows;
         const std::uint32_t urows = static_cast<std::uint32_t>(rows);
-        double* vertical = w.alloc<double>(rows);
-        double* divergence = w.alloc<double>(g.nodes);
-        double* diagonal = w.alloc<double>(rows);
-        double* off = w.alloc<double>(S.view.entries);
-        double* rhs = w.alloc<double>(rows);
-        double* start = w.alloc<double>(rows);
-        double* applied = w.alloc<double>(rows);
-        double* residual = w.alloc<double>(rows);
-        double* delta = w.alloc<double>(rows);
-        double* solved = w.alloc<double>(rows);
+        if (!S.work) S.work = std::make_unique<psgb::TracerWork>(rows, g.nodes, S.view.entries, S.ell.width);
+        psgb::TracerWork& k = *S.work;
+        double *vertical = k.vertical, *divergence = k.divergence, *diagonal = k.diagonal, *off = k.off, *rhs = k.rhs,
+               *start = k.start, *applied = k.applied, *residual = k.residual, *delta = k.delta, *solved = k.solved,
+               *off_ell = k.off_ell;
+        psgb::Scalars& sc = k.scalars;
         double* out = memory == PSGB_MEMORY_DEVICE ? tracer_out : w.alloc<double>(rows);
         const double exchange_scale = 1.0 / (transport->heat_capacity_J_kg_K * static_cast<double>(L));
         const unsigned gn = psgb::blocks_of(g.nodes), gr = psgb::blocks_of(rows);
@@ -1123,27 +1336,22 @@ int psgb_solve_implicit_tracer(psgb_planet* planet, const psgb_advection_diffusi
                                                               c0, diagonal, off, rhs, start);
         PSGB_CHECK_LAUNCH();
         S.ilu->factor(diagonal, off, 1.0, st);
-        double* off_ell = w.alloc<double>(std::size_t(S.ell.width) * rows);
         psgb::k_csr_to_ell<<<gr, psgb::kThreads, 0, st>>>(S.ell, S.view.offset, off, off_ell);
         PSGB_CHECK_LAUNCH();
-        const psgb::Op apply = [&](const double* x, double* y) {
+        const auto apply = [&](const double* x, double* y) {
             psgb::k_ell_apply<<<gr, psgb::kThreads, 0, st>>>(S.ell, off_ell, diagonal, x, y);
             PSGB_CHECK_LAUNCH();
         };
-        const psgb::Op precondition = [&](const double* x, double* y) {
-            psgb::k_copy<<<gr, psgb::kThreads, 0, st>>>(urows, x, y);
-            PSGB_CHECK_LAUNCH();
-            S.ilu->solve(y, st);
+        const psgb::Precondition precondition = [&](const double* x, double* y, const int* skip) {
+            S.ilu->solve(x, y, st, skip);
         };
         // A delta = b - A c0, from delta = 0.
         apply(start, applied);
         psgb::k_sub<<<gr, psgb::kThreads, 0, st>>>(urows, rhs, applied, residual);
         PSGB_CHECK_LAUNCH();
-        psgb::Scalars sc(w, rows);
-        const psgb::BicgWork work(w, rows);
         psgb_tracer_result r{};
-        r.iterations = psgb::bicgstab(rows, apply, precondition, residual, delta, relative_tolerance, max_iterations,
-                                      work, sc, st);
+        r.iterations = psgb::bicgstab(S.ell, off_ell, diagonal, precondition, true, residual, delta, relative_tolerance,
+                                      max_iterations, k.bicg, sc, st);
         psgb::k_tracer_solved<<<gr, psgb::kThreads, 0, st>>>(urows, start, delta, solved);
         PSGB_CHECK_LAUNCH();
         apply(solved, applied);
@@ -1263,13 +1471,13 @@ int psgb_solve_implicit_advection_diffusion(psgb_planet* planet, const psgb_adve
         psgb_advection_result out{};
         int non_monotone = 0;
         double* off_ell = w.alloc<double>(std::size_t(c.graph_ell.width) * n);
-        const psgb::Op apply = [&](const double* x, double* y) {
+        const auto apply = [&](const double* x, double* y) {
             psgb::k_ell_apply<<<gn, psgb::kThreads, 0, st>>>(c.graph_ell, off_ell, diagonal, x, y);
             PSGB_CHECK_LAUNCH();
         };
         // The V-cycle of A theta'^-1 + K on A x, divided by theta', then the block ILU of J
         // on what is left (heat_transport.cpp:1233-1249).
-        const psgb::Op precondition = [&](const double* x, double* y) {
+        const psgb::Precondition precondition = [&](const double* x, double* y, const int*) {
             psgb::k_scale_area<<<gn, psgb::kThreads, 0, st>>>(n, g.area, x, scaled);
             PSGB_CHECK_LAUNCH();
             if (psgb_multigrid_precondition(planet, PSGB_DTYPE_F64, scaled, y, PSGB_MEMORY_DEVICE, st) != PSGB_OK)
@@ -1279,7 +1487,7 @@ int psgb_solve_implicit_advection_diffusion(psgb_planet* planet, const psgb_adve
             apply(y, leftover);
             psgb::k_leftover<<<gn, psgb::kThreads, 0, st>>>(n, x, leftover);
             PSGB_CHECK_LAUNCH();
-            c.graph_ilu->solve(leftover, st);
+            c.graph_ilu->solve(leftover, leftover, st);
             psgb::k_add<<<gn, psgb::kThreads, 0, st>>>(n, leftover, y);
             PSGB_CHECK_LAUNCH();
         };
@@ -1294,8 +1502,8 @@ int psgb_solve_implicit_advection_diffusion(psgb_planet* planet, const psgb_adve
             PSGB_CHECK_LAUNCH();
             if (psgb_multigrid_set_matrix(planet, sym_diagonal, sym_off, PSGB_MEMORY_DEVICE, st) != PSGB_OK)
                 throw std::runtime_error(psgb_last_error());
-            out.linear_iterations += psgb::bicgstab(n, apply, precondition, rhs, delta, settings.cg_relative_tolerance,
-                                                    settings.max_cg_iterations, work, sc, st);
+            out.linear_iterations += psgb::bicgstab(c.graph_ell, off_ell, diagonal, precondition, false, rhs, delta,
+                                                    settings.cg_relative_tolerance, settings.max_cg_iterations, work, sc, st);
             // Backtracking on the merit (heat_transport.cpp:1255-1292).
             double step = 1.0;
             bool accepted = false;

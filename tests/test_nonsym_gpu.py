@@ -233,3 +233,65 @@ def test_tracer_and_coupled_solve_against_the_oracle_at_l5():
                                                              b, eps, phi, floor)
     assert got.consistency_residual_W_m2 <= 1e-6 and ostats[2] <= 1e-6
     assert np.max(np.abs(got.source_W_m2 - src)) <= 1e-5
+
+
+def block_ilu_reference(off, nb, diag, val, blocks, x):
+    """ILU(0) of each diagonal block, IKJ over columns in ascending order, and its solve."""
+    y = np.empty_like(x)
+    for b0, b1 in zip(blocks[:-1], blocks[1:]):
+        rows = []
+        for i in range(b0, b1):
+            row = {int(nb[k]): val[k] for k in range(off[i], off[i + 1]) if b0 <= nb[k] < b1}
+            row[i] = diag[i]
+            row = dict(sorted(row.items()))
+            for j in row:
+                if j >= i:
+                    break
+                other = rows[j - b0]
+                row[j] = row[j] / other[j]
+                for c, v in other.items():
+                    if c > j and c in row:
+                        row[c] = row[c] - row[j] * v
+            rows.append(row)
+        for i in range(b0, b1):
+            s = x[i]
+            for c, v in rows[i - b0].items():
+                if c < i:
+                    s = s - v * y[c]
+            y[i] = s
+        for i in range(b1 - 1, b0 - 1, -1):
+            s = y[i]
+            for c, v in rows[i - b0].items():
+                if c > i:
+                    s = s - v * y[c]
+            y[i] = s / rows[i - b0][i]
+    return y
+
+
+@pytest.mark.parametrize("blocks", ["one", "ragged", "halves", "many"])
+@pytest.mark.parametrize("scale", [0.0, 130.0, 900.0])
+def test_block_ilu_solve_shapes(planets, blocks, scale):
+    """Blocks of every shape, empty and one-row ones too; rows of one level in another order than
+    the matrix's; the division by the diagonal a multiplication with corrections where the
+    magnitudes are ordinary. All give the sequential elimination's bits: the operations are
+    IEEE's, in the same order."""
+    import planet_game_gb300 as pg
+
+    off, nb, _, _ = graph_of(planets["mesh"])
+    n = len(off) - 1
+    rng = np.random.default_rng(5)
+    starts = {"one": [0, n], "ragged": [0, 1, 1, 34, 200, 201, n - 65, n],
+              "halves": [0, n // 2, n], "many": list(np.linspace(0, n, 78).astype(int))}[blocks]
+    two = np.exp2(rng.uniform(-1.0, 1.0, n) * scale) if scale < 500 else np.full(n, 1.0)
+    val = -rng.uniform(0.1, 1.0, len(nb))
+    diag = rng.uniform(6.5, 9.0, n) * rng.choice([-1.0, 1.0], n)
+    rows = np.repeat(np.arange(n), np.diff(off))
+    diag, val = diag * two, val * two[rows]
+    x = rng.standard_normal(n)
+    x[rng.integers(0, n, n // 4)] = 0.0
+    x[rng.integers(0, n, 9)] = -0.0
+    if scale > 500:
+        x = x * 2.0 ** -scale
+    got = pg.IncompleteLU(off, nb, diag, val, starts).solve(x)
+    want = block_ilu_reference(off, nb, diag, val, starts, x)
+    assert np.array_equal(got.view(np.int64), want.view(np.int64))
