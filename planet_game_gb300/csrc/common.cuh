@@ -96,4 +96,38 @@ __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a,
 __device__ __forceinline__ double dmul(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ double dsub(double a, double b) { return __dsub_rn(a, b); }
 
+// An SM starts an FP64 instruction of a warp every 19 cycles; a comparison or a conversion of a
+// double counts as one, whole-number work beside them is free.
+
+// The reciprocal that divide_by() takes: RN(1/d) of a d of ordinary size, else 0.
+__device__ __forceinline__ double reciprocal_of(double d) {
+    return fabs(d) > 0x1p-100 && fabs(d) < 0x1p100 ? __ddiv_rn(1.0, d) : 0.0;
+}
+
+// s / d, correctly rounded, in five operations on r = reciprocal_of(d) (Markstein, IBM J. Res.
+// Dev. 34, 1990: with r = RN(1/d) and a quotient q within one unit in the last place,
+// RN(q + r (s - d q)) is RN(s/d); one such step from q = RN(s r) gives that quotient, the next
+// rounds it). A dividend so large or small that a remainder could leave the range is divided.
+__device__ __forceinline__ double divide_by(double s, double d, double r) {
+    const std::uint32_t high = static_cast<std::uint32_t>(__double2hiint(s)) & 0x7fffffffu;
+    constexpr std::uint32_t low = (1023u - 800u) << 20, span = 1600u << 20;   // 2^-800 <= |s| < 2^800
+    if (__double2hiint(r) != 0 && high - low < span) {
+        double q = __dmul_rn(s, r);
+        q = __fma_rn(__fma_rn(-d, q, s), r, q);
+        return __fma_rn(__fma_rn(-d, q, s), r, q);
+    }
+    if (__double2hiint(r) != 0 && (high | static_cast<std::uint32_t>(__double2loint(s))) == 0u) return __dmul_rn(s, r);
+    return __ddiv_rn(s, d);
+}
+
+// A float as a double, put together from its bits; zero, subnormals, infinities and NaN are converted.
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ double widen(float v) {
+    const std::uint32_t u = __float_as_uint(v), exponent = u & 0x7f800000u;
+    if (exponent - 0x00800000u < 0x7f000000u)
+        return __hiloint2double(static_cast<int>((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))),
+                                static_cast<int>(u << 29));
+    return static_cast<double>(v);
+}
+
 }  // namespace psgb

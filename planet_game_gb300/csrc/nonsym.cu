@@ -18,6 +18,7 @@
 // Compiled without FMA contraction: every expression rounds as the reference's does.
 #include "../../include/planetsim_gb300.h"
 #include "capi_internal.hpp"
+#include "common.cuh"
 #include "host/ilu_pattern.hpp"
 
 #include <cuda_runtime.h>
@@ -124,10 +125,8 @@ __global__ void __launch_bounds__(kIluThreads) k_ilu_solve(IluView v, double* __
 // on the way back a division. An SM starts an FP64 instruction of a warp every 19 cycles, the
 // same warp's next one after 66, and one lane costs what 32 do: the levels are bound by these
 // instructions. So a warp's rows have the same number of couplings and the terms that none of them
-// has are not issued (as selections, every row paid for eight); the division by the diagonal is
-// five operations on its stored reciprocal (Markstein, IBM J. Res. Dev. 34, 1990: with r = RN(1/d)
-// and a quotient q within one unit in the last place, RN(q + r (s - d q)) is RN(s/d); one such step
-// from q = RN(s r) gives that quotient, the next rounds it); and a level's records are
+// has are not issued (as selections, every row paid for eight); the division by the diagonal takes
+// its stored reciprocal; and a level's records are
 // loaded, one value a plane, while the level before computes. A pair of SMs a block, half of each level's rows on either, was slower: its barrier and
 // the store to the partner take 400 to 900 cycles a level, as much as the halves save.
 // Ten layers on 10,242 nodes, 41 blocks of 2,560 rows in 23 levels each way: 51 us a
@@ -158,7 +157,7 @@ __global__ void k_ilu_pack(std::uint32_t rows, IluShared s, const double* __rest
         s.up.val[k * rows + idx] = k < s.up.head[idx] >> 16 ? value[s.up.q[idx * 8 + k]] : 0.0;
     }
     const double d = value[s.up.dq[idx]];
-    s.up.diag[idx] = make_double2(d, fabs(d) > 0x1p-100 && fabs(d) < 0x1p100 ? 1.0 / d : 0.0);
+    s.up.diag[idx] = make_double2(d, reciprocal_of(d));
 }
 
 // A row's record as it is loaded; nothing here is looked at before its level.
@@ -185,21 +184,6 @@ __device__ __forceinline__ double subtract_terms(const Rec& c, const double* xs,
 #pragma unroll
     for (int k = 0; k < N; ++k) sum -= p[k];
     return sum;
-}
-
-// s / d, correctly rounded, from r = RN(1/d) of a diagonal of ordinary size (0: divide). The
-// magnitude is looked at in whole numbers: a comparison of doubles takes the FP64 unit as long as
-// a product.
-__device__ __forceinline__ double quotient(double s, double d, double r) {
-    const std::uint32_t high = static_cast<std::uint32_t>(__double2hiint(s)) & 0x7fffffffu;
-    constexpr std::uint32_t low = (1023u - 800u) << 20, span = 1600u << 20;   // 2^-800 <= |s| < 2^800
-    if (__double2hiint(r) != 0 && high - low < span) {
-        double q = s * r;
-        q = __fma_rn(__fma_rn(-d, q, s), r, q);
-        return __fma_rn(__fma_rn(-d, q, s), r, q);
-    }
-    if (__double2hiint(r) != 0 && (high | static_cast<std::uint32_t>(__double2loint(s))) == 0u) return s * r;
-    return s / d;
 }
 
 constexpr unsigned kIluSharedThreads = 512;   // the widest level the shared-memory solve takes
@@ -258,7 +242,7 @@ __global__ void __launch_bounds__(kIluSharedThreads, 1) k_ilu_solve_shared(IluSh
             default: sum = subtract_terms<8>(c, xs, sum); break;
         }
         if (on) {
-            if (lv >= lo_levels) sum = quotient(sum, c.diag.x, c.diag.y);
+            if (lv >= lo_levels) sum = divide_by(sum, c.diag.x, c.diag.y);
             xs[row] = sum;
         }
         __syncthreads();

@@ -9,6 +9,9 @@ namespace psgb {
 // Sub-step-mean insolation per cell (insolation.cu), FP32 out.
 void launch_substep_insolation(const DevMesh& m, const InsolationNodes& nodes, float* out, cudaStream_t st);
 
+// Fills m.rdist, m.rarea and m.rdet; returns when they are there.
+void fill_reciprocals(const DevMesh& m);
+
 template <typename T>
 void launch_laplacian(const DevMesh& m, const T* in, T* out, cudaStream_t st);
 template <typename T>

@@ -107,6 +107,9 @@ struct DevMesh {
     double* area = nullptr;            // [P] mesh cell areas; 1 in padding rows
     double* graph_area = nullptr;      // [P] the transport graph's node areas (differ when agglomerated)
     double* gm = nullptr;              // [4][P] m_ee, m_en, m_nn, det of the LSQ gradient
+    double* rdist = nullptr;           // [6][P] dist's, area's and det's reciprocals, for divisions by them
+    double* rarea = nullptr;           // [P]
+    double* rdet = nullptr;            // [P]
     double* edge_length = nullptr;     // [E]
     double* latitude = nullptr;        // [2][P] sin and cos of the cell centre's latitude
     // agglomerated planets: fine cells -> nodes

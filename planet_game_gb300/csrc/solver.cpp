@@ -7,6 +7,7 @@
 // solve_newton_system/GraphMultigrid (sim/planet/surface/heat_transport.cpp:337-429,
 // 545-577); a many-planet batch solves uneven planets with the same launches.
 #include "solver.hpp"
+#include "operators.hpp"
 
 #include "kernels.hpp"
 #include "coarse_tail.hpp"
@@ -176,6 +177,10 @@ void upload_planet(Planet& planet_ref) {
         d.latitude = planet->store.upload(latitude);
     }
     d.edge_length = planet->store.upload(m.edge_length_m);
+    d.rdist = planet->store.alloc<double>(6 * P);
+    d.rarea = planet->store.alloc<double>(P);
+    d.rdet = planet->store.alloc<double>(P);
+    fill_reciprocals(d);
     planet->uploaded = true;
 }
 

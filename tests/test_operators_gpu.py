@@ -151,3 +151,66 @@ def test_insolation_kernel_on_device_memory(meshes):
     m.substep_mean_insolation_gpu(3, out)
     host = m.substep_mean_insolation(3)
     assert np.all(np.abs(out.cpu().numpy() - host) <= np.spacing(np.abs(host).astype(np.float32)))
+
+
+@pytest.mark.parametrize("kind", ["ordinary", "constant", "huge", "tiny", "special"])
+@pytest.mark.parametrize("dtype", [np.float64, np.float32])
+def test_operators_over_the_whole_range_of_a_field(meshes, kind, dtype):
+    """Divisions by stored reciprocals, fields widened from their bits: against the same formulas
+    in numpy. 64-bit fields give its bits (the Laplacian's and the gradient's mesh factors are the
+    kernels' own roundings, so those two to 4 parts in 2^53 of the largest term); 32-bit ones are
+    within an ulp of 32 bits and the like. Infinities and NaN come out where they do there."""
+    import planet_game_gb300 as pg
+
+    m = meshes(3)
+    a = m.arrays()
+    n, off = m.cell_count, np.append(a["edge_offset"], m.directed_edge_count).astype(np.int64)
+    rng = np.random.default_rng(17)
+    top = 1e150 if dtype is np.float64 else 1e30
+    scale = {"huge": top, "tiny": 1 / top}.get(kind, 1.0)
+    make = lambda k: (np.full(k, 3.25) if kind == "constant" else rng.standard_normal(k) * scale).astype(dtype)
+    phi, flux = make(n), make(m.edge_count)
+    if kind == "special":
+        for f in (phi, flux):
+            f[rng.integers(0, len(f), 40)] = 0.0
+            f[rng.integers(0, len(f), 40)] = -0.0
+            f[200:210] = np.finfo(dtype).smallest_subnormal
+            f[np.nonzero(np.diff(off) == 6)[0][[5, 77, 150]]] = np.inf, -np.inf, np.nan
+    rows = np.repeat(np.arange(n), np.diff(off))
+    nb, edge = a["neighbor"].astype(np.int64), a["edge"].astype(np.int64)
+    area, length, dist = a["area_m2"], a["edge_length_m"], a["edge_distance_m"]
+    east, north = a["normal_east"].astype(np.float64), a["normal_north"].astype(np.float64)
+    wide, f64 = phi.astype(np.float64), flux.astype(np.float64)
+    with np.errstate(all="ignore"):
+        def total(terms):   # in slot order
+            out = np.zeros(n)
+            for j in range(6):
+                has = np.diff(off) > j
+                out[has] = out[has] + terms[off[:-1][has] + j]
+            return out
+        outward = np.where(a["edge_first"].astype(np.int64)[edge] == rows, f64[edge], -f64[edge])
+        div_terms = outward * length[edge]
+        div = total(div_terms) / area
+        lap_terms = (wide[nb] - wide[rows]) * (length[edge] / dist[edge])
+        lap = total(lap_terms) / area
+        slope = (wide[nb] - wide[rows]) / dist[edge]
+        ee, en, nn = total(east * east), total(east * north), total(north * north)
+        re, rn, det = total(slope * east), total(slope * north), ee * nn - en * en
+        grad = (nn * re - en * rn) / det, (ee * rn - en * re) / det
+        size = {"lap": total(np.abs(lap_terms)) / area, "div": total(np.abs(div_terms)) / area,
+                "grad": (np.abs(nn) + np.abs(en) + np.abs(ee)) * total(np.abs(slope)) / np.abs(det)}
+    eps = 2.0 ** -52 if dtype is np.float64 else 2.0 ** -23
+    got = pg.divergence(m, flux)
+    if dtype is np.float64:
+        assert np.array_equal(got.view(np.int64)[~np.isnan(div)], div.view(np.int64)[~np.isnan(div)])
+    for g, want, s in ((got, div, size["div"]), (pg.laplacian(m, phi), lap, size["lap"]),
+                       *((g, w, size["grad"]) for g, w in zip(pg.gradient(m, phi), grad))):
+        assert np.array_equal(np.isnan(g), np.isnan(want))
+        with np.errstate(over="ignore", under="ignore"):
+            want = want.astype(dtype)
+        ends = ~np.isfinite(want)
+        assert np.array_equal(g[ends], want[ends], equal_nan=True)
+        f = ~ends
+        tiniest = float(np.finfo(dtype).smallest_subnormal)
+        bound = 4 * 2.0 ** -52 * s[f] + (eps * np.abs(want[f]) + tiniest if dtype is np.float32 else 0.0)
+        assert np.all(np.abs(g[f].astype(np.float64) - want[f].astype(np.float64)) <= bound)
