@@ -214,3 +214,28 @@ def test_operators_over_the_whole_range_of_a_field(meshes, kind, dtype):
         tiniest = float(np.finfo(dtype).smallest_subnormal)
         bound = 4 * 2.0 ** -52 * s[f] + (eps * np.abs(want[f]) + tiniest if dtype is np.float32 else 0.0)
         assert np.all(np.abs(g[f].astype(np.float64) - want[f].astype(np.float64)) <= bound)
+
+
+def test_calls_follow_torchs_current_stream(meshes):
+    import torch
+
+    import planet_game_gb300 as pg
+    from planet_game_gb300 import api
+
+    assert api._current_stream() == torch.cuda.current_stream().cuda_stream
+    side = torch.cuda.Stream()
+    m = meshes(5)
+    phi = torch.from_numpy(np.random.default_rng(3).standard_normal(m.cell_count)).cuda()
+    want = pg.laplacian(m, phi)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        assert api._current_stream() == side.cuda_stream
+        late = torch.zeros_like(phi)
+        late.copy_(phi)             # the operator below has to run after it
+        got = pg.laplacian(m, late)
+    side.synchronize()
+    assert torch.equal(got, want)
+    with pytest.raises(ValueError, match="contiguous CUDA"):
+        pg.gradient(m, phi.cpu())
+    with pytest.raises(ValueError, match="contiguous CUDA"):
+        pg.divergence(m, phi.repeat_interleave(2)[::2])
