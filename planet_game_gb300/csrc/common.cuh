@@ -68,28 +68,6 @@ __device__ __forceinline__ T warp_max(T v) {
     return v;
 }
 
-// Sum over a 256-thread block in fixed order; result in thread 0.
-// `scratch` holds 8 values per accumulated quantity.
-template <typename T, int N>
-__device__ __forceinline__ void block_sum256(T (&v)[N], T (*scratch)[8]) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int q = 0; q < N; ++q) {
-        T w = warp_sum(v[q]);
-        if (lane == 0) scratch[q][warp] = w;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-#pragma unroll
-        for (int q = 0; q < N; ++q) {
-            T s = scratch[q][0];
-#pragma unroll
-            for (int w = 1; w < 8; ++w) s += scratch[q][w];
-            v[q] = s;
-        }
-    }
-}
-
 // Double precision add/multiply that the compiler may not fuse into an FMA, for
 // sums whose rounding must match the reference's sequential CPU loops.
 __device__ __forceinline__ double dadd(double a, double b) { return __dadd_rn(a, b); }

@@ -24,6 +24,7 @@
 #include "common.cuh"
 #include "profile.hpp"
 #include "operators.hpp"
+#include "phases.cuh"
 
 namespace psgb {
 namespace {
@@ -208,7 +209,7 @@ __global__ void k_step_finish(std::uint32_t P, const std::int32_t* __restrict__ 
     // columns, weights (and per-entry conductances), area, T, T0, S in; H, T_new out
     if (bytes != nullptr && threadIdx.x == 0)
         atomicAdd(bytes, (edge_conductance != nullptr ? 168ull : 120ull) * static_cast<unsigned>(tile_rows[tile]));
-    double v[6] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+    double v[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};   // six, and two zeros that fill up the tree
     if (threadIdx.x < tile_rows[tile]) {
         const double own = t[row];
         double sum = 0.0;
@@ -238,8 +239,7 @@ __global__ void k_step_finish(std::uint32_t P, const std::int32_t* __restrict__ 
         v[4] = fabs(v[3]);
         v[5] = dmul(a, __ddiv_rn(dsub(tn, t0[row]), s));
     }
-    __shared__ double scratch[6][8];
-    block_sum256<double, 6>(v, scratch);
+    ph::group_sum<double, 8>(v, 0, threadIdx.x);
     if (threadIdx.x == 0) {
 #pragma unroll
         for (int q = 0; q < 6; ++q) partial[tile * 8 + q] = v[q];

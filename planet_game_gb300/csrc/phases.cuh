@@ -129,7 +129,10 @@ __device__ __forceinline__ void warp_sum_halving(const A (&v)[N], int l32, A& mi
 }
 
 // Sum of N values over the 256 threads of a group, each value in its own fixed tree
-// (warp butterflies, then the eight warp sums in order); results in lane 0.
+// (warp butterflies, then the eight warp sums in order, a lane a value); results in lane 0.
+// One lane adding up all values in turn took 7 N FP64 instructions of 66 cycles each before a
+// block could end, every one as dear as a whole warp's: 655,362 rows in 64 bits, hot, k_bicg_x
+// (8 sums a block) 19.9 us then, 17.7 now, k_bicg_t 22.1 and 19.8, k_step_finish 105 and 72.
 template <typename A, int N>
 __device__ __forceinline__ void group_sum(A (&v)[N], int gid, int lane) {
     __shared__ A scratch[kGroups][N][8];
@@ -148,14 +151,16 @@ __device__ __forceinline__ void group_sum(A (&v)[N], int gid, int lane) {
         }
     }
     group_sync(gid);
-    if (lane == 0) {
+    static_assert(N <= 32, "a lane a value");
+    if (w == 0) {
+        A s = A(0);
+        if (lane < N) {
+            s = scratch[gid][lane][0];
 #pragma unroll
-        for (int q = 0; q < N; ++q) {
-            A s = scratch[gid][q][0];
-#pragma unroll
-            for (int k = 1; k < 8; ++k) s += scratch[gid][q][k];
-            v[q] = s;
+            for (int k = 1; k < 8; ++k) s += scratch[gid][lane][k];
         }
+#pragma unroll
+        for (int q = 0; q < N; ++q) v[q] = __shfl_sync(0xffffffffu, s, q);
     }
     group_sync(gid);
 }
