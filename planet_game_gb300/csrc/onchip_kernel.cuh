@@ -263,12 +263,6 @@ __device__ void load_dense(const Block& k, const OnchipArgs<T>& a, int inst) {
     for (int i = k.tid; i < rows * n; i += k.threads) dst[i] = __ldcg(&src[i]);
 }
 
-// The damped update of a row (phases.cuh `smooth`): s = b - O x, xo the row's iterate.
-template <typename T>
-__device__ __forceinline__ T jacobi(T inv, T s, T xo, T omega) {
-    return omega == T(1) ? prod(inv, s) : fma_(omega, fma_(inv, s, -xo), xo);
-}
-
 // ---- the V-cycle as a list of phases ------------------------------------------------------------
 //
 // The code of a phase stands once and the cycle walks a list of phases, one cluster barrier
@@ -516,7 +510,7 @@ __device__ __forceinline__ void coarse_phase(const Block& k, const Phase& p, std
         if (kind == kResidual) s = fnma(h.m.diagonal(), xo, s);
 #pragma unroll
         for (int j = 0; j < kCoarseWidth; ++j) s = fnma(h.m.v[j], g[j], s);
-        if (kind != kResidual) s = jacobi(h.m.inverse(), s, xo, omega);
+        if (kind != kResidual) s = ph::sweep_update(xo, omega, h.m.inverse(), s);
         k.at<T>(p.dst)[i] = s;
     }
 }
@@ -746,7 +740,7 @@ struct Solve {
                         T s = residual ? fnma(m.diagonal(), xo, b[r]) : b[r];
 #pragma unroll
                         for (int j = 0; j < 6; ++j) s = fnma(m.v[j], g[j], s);
-                        if (!residual) s = jacobi(m.inverse(), s, xo, omega);
+                        if (!residual) s = ph::sweep_update(xo, omega, m.inverse(), s);
                         if (my.on[r]) k.at<T>(dst)[my.row[r]] = s;
                     });
                 }

@@ -290,6 +290,10 @@ __device__ __forceinline__ bool running(const InstanceScalars& s) { return s.sta
 __device__ __forceinline__ float prod(float a, float b) { return __fmul_rn(a, b); }
 __device__ __forceinline__ double prod(double a, double b) { return __dmul_rn(a, b); }
 
+// 1, by its bits: a comparison of doubles takes the FP64 unit as long as a product.
+__device__ __forceinline__ bool is_one(float v) { return v == 1.0f; }
+__device__ __forceinline__ bool is_one(double v) { return __double2hiint(v) == 0x3ff00000 && __double2loint(v) == 0; }
+
 // The block-local sweep's arithmetic spelled out, so that every kernel sweeping a tile
 // block-locally (the kernel schedule, the coarse tails, the block step of many right-hand
 // sides) forms the same bits whatever the compiler would fuse: s - a v as one fused
@@ -301,7 +305,20 @@ __device__ __forceinline__ float jacobi_update(float xo, float omega, float inv,
     return omega == 1.0f ? __fmul_rn(inv, s) : __fmaf_rn(omega, __fsub_rn(__fmul_rn(inv, s), xo), xo);
 }
 __device__ __forceinline__ double jacobi_update(double xo, double omega, double inv, double s) {
-    return omega == 1.0 ? __dmul_rn(inv, s) : __fma_rn(omega, __dsub_rn(__dmul_rn(inv, s), xo), xo);
+    const bool plain = is_one(omega);
+    return __fma_rn(omega, __dsub_rn(__dmul_rn(inv, s), plain ? 0.0 : xo), plain ? -0.0 : xo);
+}
+
+// The update of a whole sweep, as the compiler fuses it: x + omega (D^-1 s - x), undamped D^-1 s.
+// In 64 bits two FP64 instructions whichever it is. Written as a choice of results, the compiler
+// issues both sides' and the comparison, four of a row's ten; with zeros of the right sign in the
+// places of x the undamped update comes out of the damped one's instructions bit for bit.
+__device__ __forceinline__ float sweep_update(float xo, float omega, float inv, float s) {
+    return omega == 1.0f ? __fmul_rn(inv, s) : __fmaf_rn(omega, __fmaf_rn(inv, s, -xo), xo);
+}
+__device__ __forceinline__ double sweep_update(double xo, double omega, double inv, double s) {
+    const bool plain = is_one(omega);
+    return __fma_rn(omega, __fma_rn(inv, s, plain ? -0.0 : -xo), plain ? -0.0 : xo);
 }
 
 __device__ __forceinline__ bool finite(double v) { return isfinite(v); }
@@ -472,12 +489,7 @@ __device__ void smooth(const LevelView<T>& lv, int t0, int lane, const T* PSGB_P
         T s = b[row];
 #pragma unroll
         for (int j = 0; j < W; ++j) s -= lv.vd[j * P + row] * x[col[j]];
-        if (omega == T(1)) {
-            out[k] = lv.inv[row] * s;
-        } else {
-            const T xo = x[row];
-            out[k] = xo + omega * (lv.inv[row] * s - xo);
-        }
+        out[k] = sweep_update(is_one(omega) ? T(0) : x[row], omega, lv.inv[row], s);
     }
 #pragma unroll
     for (int k = 0; k < R; ++k) {
@@ -661,18 +673,24 @@ __device__ void prolong_smooth(const LevelView<T>& lv, int t0, int lane, const s
     for (int k = 0; k < R; ++k) {
         const int row = ts.tile[k] * kTile + lane;
         const ColumnsOf col = columns_of(lv, ts.tile[k], row);
-        T s = b[row];
+        T s = b[row], xo = T(0);
+        // a correction taken as it is (times 1, the same bits) has a loop of its own
+        if (is_one(lv.correction)) {
 #pragma unroll
-        for (int j = 0; j < W; ++j) {
-            const int c = col[j];
-            s -= lv.vd[j * P + row] * (x[c] + prod(lv.correction, e[agg[c]]));
-        }
-        if (omega == T(1)) {
-            out[k] = lv.inv[row] * s;
+            for (int j = 0; j < W; ++j) {
+                const int c = col[j];
+                s -= lv.vd[j * P + row] * (x[c] + e[agg[c]]);
+            }
+            if (!is_one(omega)) xo = x[row] + e[agg[row]];
         } else {
-            const T xo = x[row] + prod(lv.correction, e[agg[row]]);
-            out[k] = xo + omega * (lv.inv[row] * s - xo);
+#pragma unroll
+            for (int j = 0; j < W; ++j) {
+                const int c = col[j];
+                s -= lv.vd[j * P + row] * (x[c] + prod(lv.correction, e[agg[c]]));
+            }
+            if (!is_one(omega)) xo = x[row] + prod(lv.correction, e[agg[row]]);
         }
+        out[k] = sweep_update(xo, omega, lv.inv[row], s);
     }
 #pragma unroll
     for (int k = 0; k < R; ++k) {
