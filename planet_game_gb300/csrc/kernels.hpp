@@ -21,6 +21,10 @@ struct InstanceScalars {
     int refinements;
     int inner_total;     // Krylov iterations summed over refinements
     int first;           // PCG: first iteration
+    // alpha, omega and beta as 32-bit solves take them, rounded once where they are set: a thread's
+    // own conversion takes the FP64 unit as long as a product, which made up half of the 32-bit
+    // vector kernels' time
+    float alpha32, omega32, beta32, unused;
 };
 
 // Tile word: planet (bits 0-21), valid rows 0..256 (bits 22-30), smooths here (bit 31).

@@ -614,7 +614,7 @@ __global__ void k_bicg_p(LevelView<T> L, const T* __restrict__ r, const T* __res
     const TileInfo ti = tile_info(L.tile_meta, tile);
     count(L.bytes, static_cast<unsigned long long>(ti.rows) * (sizeof(T) + 5ull * kRhs * sizeof(T)));
     if (ti.rows == 0 || !ph::running(sc[lane])) return;
-    const T beta = T(sc[lane].beta), omega = T(sc[lane].omega);
+    const T beta = ph::beta_of<T>(sc[lane]), omega = ph::omega_of<T>(sc[lane]);
     for (int g = 0; g < 8; ++g) {
         T pv[4], zv[4];
 #pragma unroll
@@ -672,7 +672,7 @@ __global__ void k_bicg_s(LevelView<T> L, const T* __restrict__ r, const T* __res
     const int tile = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const TileInfo ti = tile_info(L.tile_meta, tile);
     const bool on = ti.rows > 0 && ph::running(ctx.sc[lane]);
-    const T alpha = T(ctx.sc[lane].alpha);
+    const T alpha = ph::alpha_of<T>(ctx.sc[lane]);
     count(L.bytes, static_cast<unsigned long long>(ti.rows) * (sizeof(T) + 4ull * kRhs * sizeof(T)));
     T run[8];
     for (int g = 0; g < 8; ++g) {
@@ -739,7 +739,7 @@ __global__ void k_bicg_x(LevelView<T> L, const T* __restrict__ phat, const T* __
     const InstanceScalars& sc = ctx.sc[lane];
     const bool on = ti.rows > 0 && ph::running(sc);
     const bool half = sc.half_done != 0;
-    const T alpha = T(sc.alpha), omega = T(sc.omega);
+    const T alpha = ph::alpha_of<T>(sc), omega = ph::omega_of<T>(sc);
     count(L.bytes, static_cast<unsigned long long>(ti.rows) * 8ull * kRhs * sizeof(T));
     T run0[8], run1[8];
     for (int g = 0; g < 8; ++g) {

@@ -786,11 +786,11 @@ struct Solve {
             const std::uint32_t first = L.starts_in_x ? o_hat : L.o_y;
             T m[R];
             if (half == 0) {
-                const T beta = T(red.s.beta), om = T(red.s.omega);
+                const T beta = ph::beta_of<T>(red.s), om = ph::omega_of<T>(red.s);
 #pragma unroll
                 for (int r = 0; r < R; ++r) m[r] = p[r] = fma_(beta, fnma(om, v[r], p[r]), rr[r]);
             } else {
-                const T alpha = T(red.s.alpha);
+                const T alpha = ph::alpha_of<T>(red.s);
 #pragma unroll
                 for (int r = 0; r < R; ++r) {
                     m[r] = rr[r] = fnma(alpha, v[r], rr[r]);   // s
@@ -809,7 +809,7 @@ struct Solve {
                 if (red.s.status != kRunning) break;
                 if (red.s.half_done) {
                     // converged at s: x += alpha p_hat closes the iteration
-                    const T alpha = T(red.s.alpha);
+                    const T alpha = ph::alpha_of<T>(red.s);
 #pragma unroll
                     for (int r = 0; r < R; ++r) x[r] = fma_(alpha, k.at<T>(a.o_phat)[my.row[r]], x[r]);
                     __syncthreads();
@@ -840,7 +840,7 @@ struct Solve {
             }
             reduce(q2, ph::kFinBicgT);
             if (red.s.status != kRunning) break;
-            const T alpha = T(red.s.alpha), w = T(red.s.omega);
+            const T alpha = ph::alpha_of<T>(red.s), w = ph::omega_of<T>(red.s);
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 x[r] = add_(x[r], fma_(alpha, k.at<T>(a.o_phat)[my.row[r]], prod(w, k.at<T>(a.o_shat)[my.row[r]])));

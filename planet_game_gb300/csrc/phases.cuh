@@ -743,12 +743,32 @@ __device__ void dense_block(const DenseTask<T>& task, unsigned k, int lane, cons
         atomicAdd(task.bytes, static_cast<unsigned long long>(task.dense.size[blk.x] + 1) * sizeof(T));
 }
 
+// The coefficients in a solve's type, and setting them.
+template <typename T>
+__device__ __forceinline__ T alpha_of(const InstanceScalars& s) {
+    if constexpr (sizeof(T) == 8) return s.alpha; else return s.alpha32;
+}
+template <typename T>
+__device__ __forceinline__ T omega_of(const InstanceScalars& s) {
+    if constexpr (sizeof(T) == 8) return s.omega; else return s.omega32;
+}
+template <typename T>
+__device__ __forceinline__ T beta_of(const InstanceScalars& s) {
+    if constexpr (sizeof(T) == 8) return s.beta; else return s.beta32;
+}
+__device__ inline void set_alpha(InstanceScalars& s, double v) { s.alpha = v; s.alpha32 = static_cast<float>(v); }
+__device__ inline void set_omega(InstanceScalars& s, double v) { s.omega = v; s.omega32 = static_cast<float>(v); }
+__device__ inline void set_beta(InstanceScalars& s, double v) { s.beta = v; s.beta32 = static_cast<float>(v); }
+
 // ---- scalar steps: one planet, once its sums are complete (ticket or finish launch) ----
 
 __device__ inline void finish_bicg_init(InstanceScalars& s, const double* sum, double tol, int max_it) {
     s.b_norm = sqrt(sum[0]);
     s.target = fmax(tol * s.b_norm, 0.5 * s.outer_target);
-    s.rho = sum[0]; s.alpha = 1.0; s.omega = 1.0; s.beta = 0.0;
+    s.rho = sum[0];
+    set_alpha(s, 1.0);
+    set_omega(s, 1.0);
+    set_beta(s, 0.0);
     s.iterations = 0; s.half_done = 0; s.max_iterations = max_it; s.first = 1;
     s.r_norm = s.b_norm;
     s.status = !finite(s.b_norm) ? kNonFinite : (s.b_norm > 0.0 ? kRunning : kConverged);
@@ -758,7 +778,7 @@ __device__ inline void finish_bicg_init(InstanceScalars& s, const double* sum, d
 __device__ inline void finish_bicg_v(InstanceScalars& s, const double* sum) {
     if (!finite(sum[0])) { s.status = kNonFinite; return; }
     if (sum[0] == 0.0) { s.status = kBreakdown; return; }
-    s.alpha = s.rho / sum[0];
+    set_alpha(s, s.rho / sum[0]);
 }
 
 // ||s||: converged at s -> the iteration finishes with x += alpha p_hat.
@@ -771,7 +791,7 @@ __device__ inline void finish_bicg_s(InstanceScalars& s, const double* sum) {
 
 // omega = (t.s) / (t.t)
 __device__ inline void finish_bicg_t(InstanceScalars& s, const double* sum) {
-    s.omega = sum[0] > 0.0 ? sum[1] / sum[0] : 0.0;
+    set_omega(s, sum[0] > 0.0 ? sum[1] / sum[0] : 0.0);
     if (!finite(s.omega)) s.status = kNonFinite;
 }
 
@@ -788,7 +808,7 @@ __device__ inline void finish_bicg_x(InstanceScalars& s, const double* sum) {
     if (s.r_norm <= s.target) { s.status = kConverged; return; }
     const double rho_next = sum[1];
     if (rho_next == 0.0 || s.omega == 0.0) { s.status = kBreakdown; return; }
-    s.beta = rho_next / s.rho * (s.alpha / s.omega);
+    set_beta(s, rho_next / s.rho * (s.alpha / s.omega));
     s.rho = rho_next;
     if (s.iterations >= s.max_iterations) s.status = kCap;
 }
@@ -798,7 +818,9 @@ __device__ inline void finish_pcg_init(InstanceScalars& s, const double* sum, do
     s.target = fmax(tol * s.b_norm, 0.5 * s.outer_target);
     s.r_norm = s.b_norm;
     s.iterations = 0; s.half_done = 0; s.max_iterations = max_it; s.first = 1;
-    s.rho = 0.0; s.beta = 0.0; s.alpha = 0.0;
+    s.rho = 0.0;
+    set_beta(s, 0.0);
+    set_alpha(s, 0.0);
     s.status = !finite(s.b_norm) ? kNonFinite : (s.b_norm > 0.0 ? kRunning : kConverged);
 }
 
@@ -806,7 +828,7 @@ __device__ inline void finish_pcg_init(InstanceScalars& s, const double* sum, do
 __device__ inline void finish_pcg_rz(InstanceScalars& s, const double* sum) {
     if (!finite(sum[0])) { s.status = kNonFinite; return; }
     if (!(sum[0] > 0.0)) { s.status = s.first ? kConverged : kBreakdown; return; }
-    s.beta = s.first ? 0.0 : sum[0] / s.rho;
+    set_beta(s, s.first ? 0.0 : sum[0] / s.rho);
     s.rho = sum[0];
     s.first = 0;
 }
@@ -815,7 +837,7 @@ __device__ inline void finish_pcg_rz(InstanceScalars& s, const double* sum) {
 __device__ inline void finish_pcg_q(InstanceScalars& s, const double* sum) {
     if (!finite(sum[0])) { s.status = kNonFinite; return; }
     if (!(sum[0] > 0.0)) { s.status = kBreakdown; return; }
-    s.alpha = s.rho / sum[0];
+    set_alpha(s, s.rho / sum[0]);
 }
 
 // ||r|| -> converged?
@@ -951,7 +973,7 @@ __device__ void bicg_p(const LevelView<T>& lv, int t0, int lane, const T* PSGB_P
 #pragma unroll
     for (int k = 0; k < R; ++k) {
         const int row = ts.tile[k] * kTile + lane;
-        const T beta = T(sc[ts.inst[k]].beta), omega = T(sc[ts.inst[k]].omega);
+        const T beta = beta_of<T>(sc[ts.inst[k]]), omega = omega_of<T>(sc[ts.inst[k]]);
         pv[k] = r[row] + beta * (p[row] - omega * v[row]);
         zv[k] = omega_j * lv.inv[row] * pv[k];
     }
@@ -1015,7 +1037,7 @@ __device__ void bicg_s(const LevelView<T>& lv, int t0, int gid, int lane, const 
 #pragma unroll
     for (int k = 0; k < R; ++k) {
         const int row = ts.tile[k] * kTile + lane;
-        const T alpha = T(ctx.sc[ts.inst[k]].alpha);
+        const T alpha = alpha_of<T>(ctx.sc[ts.inst[k]]);
         sv[k] = r[row] - alpha * v[row];
         zv[k] = omega_j * lv.inv[row] * sv[k];
     }
@@ -1100,7 +1122,7 @@ __device__ void bicg_x(const LevelView<T>& lv, int t0, int gid, int lane, const 
     for (int k = 0; k < R; ++k) {
         const int row = ts.tile[k] * kTile + lane;
         const InstanceScalars& sc = ctx.sc[ts.inst[k]];
-        const T alpha = T(sc.alpha), omega = T(sc.omega);
+        const T alpha = alpha_of<T>(sc), omega = omega_of<T>(sc);
         if (half[k]) {
             xv[k] = x[row] + alpha * phat[row];
             rv[k] = T(0);
@@ -1196,7 +1218,7 @@ __device__ void pcg_p(const LevelView<T>& lv, int t0, int lane, const T* PSGB_PH
     for (int k = 0; k < R; ++k) {
         if (lane >= ts.rows[k] || !on[k]) continue;
         const int row = ts.tile[k] * kTile + lane;
-        p[row] = z[row] + T(sc[ts.inst[k]].beta) * p[row];
+        p[row] = z[row] + beta_of<T>(sc[ts.inst[k]]) * p[row];
     }
 }
 
@@ -1251,7 +1273,7 @@ __device__ void pcg_xr(const LevelView<T>& lv, int t0, int gid, int lane, const 
 #pragma unroll
     for (int k = 0; k < R; ++k) {
         const int row = ts.tile[k] * kTile + lane;
-        const T alpha = T(ctx.sc[ts.inst[k]].alpha);
+        const T alpha = alpha_of<T>(ctx.sc[ts.inst[k]]);
         xn[k] = x[row] + alpha * p[row];
         rn[k] = r[row] - alpha * q_in[row];
         zn[k] = omega_j * lv.inv[row] * rn[k];
