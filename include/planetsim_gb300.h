@@ -68,7 +68,8 @@ extern "C" {
 #define PSGB_METHOD_BICGSTAB 1
 
 /* How a solve is scheduled on the GPU. */
-#define PSGB_SCHEDULE_AUTO 0        /* the library's choice: currently the kernel schedule (faster on GB300) */
+#define PSGB_SCHEDULE_AUTO 0        /* the library's choice: where a batch's planets all fit, each solved
+                                       whole on a thread-block cluster's SMs; else the kernel schedule */
 #define PSGB_SCHEDULE_KERNELS 1     /* one kernel per phase; Krylov chunks replayed as CUDA graphs */
 #define PSGB_SCHEDULE_PERSISTENT 2  /* one cooperative kernel per solve (grid barriers between phases) */
 
@@ -490,12 +491,14 @@ typedef struct psgb_tuning {
     int pre_sweeps[PSGB_MAX_LEVELS];      /* per level, 1..8 */
     int post_sweeps[PSGB_MAX_LEVELS];     /* per level, 0..8 */
     int stencil_tiles[PSGB_MAX_LEVELS];   /* tiles per thread of the stencil launches: 1 or 2 */
-    int vector_tiles[PSGB_MAX_LEVELS];    /* tiles per thread of the vector launches: 1 or 4 */
+    int vector_tiles[PSGB_MAX_LEVELS];    /* tiles per thread of the vector launches: 1 or 4
+                                             (levels of 2,432 tiles and more run 4 whichever) */
     double jacobi_omega;
     double tuned_solve_ms;                /* autotune: trial solve with the chosen settings */
     double default_solve_ms;              /* autotune: trial solve with the settings before */
     int trial_solves;                     /* autotune: solves timed */
-    int coarse_tail_level;                /* levels from this one down run one block per planet; 0: none */
+    int coarse_tail_level;                /* levels from this one down run one block per planet; 0: none
+                                             (also the default of a batch in the library's own memory) */
     int block_sweeps[PSGB_MAX_LEVELS];    /* per level: Jacobi sweeps per smoothing launch, each tile in shared
                                              memory with its neighbours in other tiles held (1..8; 1 = plain) */
     int coarse_tail_single;               /* 0: a large planet's tail runs on several co-resident blocks

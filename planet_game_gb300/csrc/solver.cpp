@@ -38,10 +38,6 @@ Batch::~Batch() {
 
 namespace {
 
-// Levels with at least this many tiles (two waves of eight 256-thread blocks on 152 SMs)
-// use multi-tile sets by default.
-constexpr std::uint32_t kSetsMinTiles = 2 * 8 * 152;
-
 // Levels whose planets hold at most this many rows each run in the coarse tail.
 constexpr std::uint32_t kTailRows = 4096;
 
@@ -510,7 +506,7 @@ static LevelView<T> make_view(const BatchLevel& L, const T* vd, const T* inv, st
     LevelView<T> v{L.rows,         L.width,        L.tiles,      L.col,
                    vd,             inv,            L.tile_inst,  L.tile_rows,
                    L.tile_sweep,   L.tile_meta,    nullptr,
-                   L.sets_stencil, L.sets_vector,  static_cast<std::uint8_t>(level)};
+                   L.sets_stencil, vector_sets(L), static_cast<std::uint8_t>(level)};
     v.scol = L.scol;
     v.tile_shift = L.tile_shift;
     v.spitch = L.spitch;

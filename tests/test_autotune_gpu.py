@@ -307,3 +307,30 @@ def test_scaled_coarse_correction_same_bits_on_every_schedule_and_meets_the_orac
     t["coarse_correction"] = 1.0
     batch.set_tuning(t)
     assert batch.tuning["coarse_correction"] == 1.0
+
+
+@pytest.mark.parametrize("precision", ["mixed", "fp64"])
+def test_vector_launches_of_large_levels(meshes, precision):
+    """Sixteen L6 planets (2,576 tiles) run four tiles a thread whichever setting they have; the
+    results and the counts are those of the planets in batches too small for that."""
+    import planet_game_gb300 as pg
+    from planet_game_gb300 import workloads as W
+
+    m = meshes(6)
+    inputs = [W.step_inputs(m, seed=k) for k in range(16)]
+    settings = {"pre_sweeps": [1, 2, 1], "post_sweeps": [1, 2, 1], "stencil_tiles": [1, 1, 1], "vector_tiles": [1, 1, 1],
+                "block_sweeps": [1, 4, 1], "jacobi_omega": 1.0}
+
+    def run(part, tiles):
+        b = pg.Batch([m] * len(part))
+        b.set_tuning(dict(settings, vector_tiles=[tiles, 1, 1]))
+        assert b.tuning["vector_tiles"][0] == tiles
+        return b.transport_step([i.t0 for i in part], [i.source for i in part], inputs[0].heat_capacity, inputs[0].dt,
+                                inputs[0].conductance, precision=precision, schedule="kernels")
+
+    out, reports = run(inputs, 1)
+    four, _ = run(inputs, 4)
+    for k in (0, 7, 15):
+        small, small_reports = run(inputs[k:k + 1], 1)
+        assert np.array_equal(out[k], small[0]) and np.array_equal(four[k], small[0])
+        assert reports[k].iterations == small_reports[0].iterations
