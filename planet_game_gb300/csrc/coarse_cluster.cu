@@ -11,6 +11,7 @@
 // the tail level's right-hand side and the iterate of its zero-start sweep; out: its final
 // iterate, as for the other tails.
 #include "coarse_tail.hpp"
+#include "host/per_device.hpp"
 #include "phases.cuh"
 #include "planet.hpp"
 #include "profile.hpp"
@@ -380,7 +381,8 @@ __global__ void __launch_bounds__(1024, 1) k_coarse_cluster(const __grid_constan
 
 template <typename T>
 unsigned cluster_tail_max_bytes() {
-    static const unsigned limit = [] {
+    static PerDevice<unsigned> limit;
+    return limit.of(current_device(), [] {
         int device = 0, optin = 0, cluster = 0;
         cudaFuncAttributes fa{};
         if (cudaGetDevice(&device) != cudaSuccess ||
@@ -397,8 +399,7 @@ unsigned cluster_tail_max_bytes() {
             return 0u;
         }
         return static_cast<unsigned>(room);
-    }();
-    return limit;
+    });
 }
 template unsigned cluster_tail_max_bytes<float>();
 template unsigned cluster_tail_max_bytes<double>();

@@ -5,6 +5,7 @@
 // memory); the dense coarsest solve gives one row to each of the planet's warps.
 #define PSGB_PHASE_RESTRICT
 #include "coarse_tail.hpp"
+#include "host/per_device.hpp"
 #include "phases.cuh"
 #include "planet.hpp"
 #include "profile.hpp"
@@ -273,8 +274,9 @@ unsigned tail_block_budget() {
 template <typename T>
 unsigned tail_shared_max_bytes() {
     // the block's opt-in shared memory less the kernel's static shared memory (its copy of
-    // the arguments, the block-local sweeps' tiles); the kernel is opted in to it once
-    static const unsigned limit = [] {
+    // the arguments, the block-local sweeps' tiles); the kernel is opted in to it once a device
+    static PerDevice<unsigned> limit;
+    return limit.of(current_device(), [] {
         int device = 0, optin = 0;
         cudaFuncAttributes fa{};
         if (cudaGetDevice(&device) != cudaSuccess ||
@@ -291,8 +293,7 @@ unsigned tail_shared_max_bytes() {
             return 0u;
         }
         return static_cast<unsigned>(room);
-    }();
-    return limit;
+    });
 }
 template unsigned tail_shared_max_bytes<float>();
 template unsigned tail_shared_max_bytes<double>();

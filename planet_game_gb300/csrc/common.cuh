@@ -22,6 +22,16 @@ namespace psgb {
 
 constexpr int kTile = 256;
 
+// The device of the calling thread (-1: none).
+inline int current_device() {
+    int device = -1;
+    if (cudaGetDevice(&device) != cudaSuccess) {
+        cudaGetLastError();
+        return -1;
+    }
+    return device;
+}
+
 // Programmatic dependent launch. Solve kernels run back to back on one stream, each
 // short; launched with launch_pdl, a kernel's blocks may be scheduled while its
 // predecessor drains. Every such kernel starts with pdl_begin(): it waits until the

@@ -13,6 +13,7 @@
 // from 2.9 to 2.1 ms with it (162 rows), a solve that assembles for every Newton step from 6.24 to
 // 6.18 (42 rows, 65 us an inverse before).
 #include "common.cuh"
+#include "host/per_device.hpp"
 #include "kernels.hpp"
 #include "phases.cuh"
 #include "profile.hpp"
@@ -118,13 +119,13 @@ std::size_t invert_bytes(int n, int cluster) {
 
 void launch_dense_invert(const DenseView& dense, int level, const LevelView<double>& lv, std::uint32_t max_rows,
                          std::uint32_t planets, double* inv64, float* inv32, cudaStream_t st) {
-    static const bool ready = [] {
+    static PerDevice<bool> ready;
+    ready.of(current_device(), [] {
         if (cudaFuncSetAttribute(k_dense_invert, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess ||
             cudaFuncSetAttribute(k_dense_invert, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
             throw std::runtime_error("dense inverse: the device cannot launch its clusters");
         return true;
-    }();
-    (void)ready;
+    });
     // As many blocks a planet as let every planet run at once (clusters of 16, 8, 4 and 2 with
     // full shared memory that are resident on 152 SMs: 7, 15, 36, 76), and as its rows need.
     const int n = static_cast<int>(max_rows);

@@ -18,6 +18,7 @@
 // the tile partials exactly as the single solve's finish does. Each right-hand side
 // therefore follows the single solve of that sub-step bit for bit.
 #include "common.cuh"
+#include "host/per_device.hpp"
 #include "kernels.hpp"
 #include "multirhs.hpp"
 #include "phases.cuh"
@@ -331,12 +332,12 @@ __global__ void __launch_bounds__(kTile) k_smooth_block(LevelView<T> L, const T*
 
 template <typename T, int W>
 void set_block_sweep_smem() {
-    static const bool done = [] {
+    static PerDevice<bool> done;
+    done.of(current_device(), [] {
         PSGB_CUDA(cudaFuncSetAttribute(k_smooth_block<T, W>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(BlockSweepSmem<T, W>::bytes)));
         return true;
-    }();
-    (void)done;
+    });
 }
 
 template <typename T, int W>

@@ -18,6 +18,7 @@
 #pragma once
 
 #define PSGB_PHASE_RESTRICT
+#include "host/per_device.hpp"
 #include "onchip.hpp"
 #include "phases.cuh"
 
@@ -989,10 +990,11 @@ KernelOf<T> kernel_of(int rows_per_thread) {
 }
 
 // Dynamic shared memory a block of the kernel may take, with the kernel's attributes set
-// (0: the device cannot launch it).
+// (0: the current device cannot launch it).
 template <typename T>
 unsigned shared_limit(int rows_per_thread) {
-    static const std::array<unsigned, 8> limits = [] {
+    static PerDevice<std::array<unsigned, 8>> limits;
+    return limits.of(current_device(), [] {
         std::array<unsigned, 8> out{};
         int device = 0, optin = 0, cluster = 0;
         if (cudaGetDevice(&device) != cudaSuccess ||
@@ -1016,8 +1018,7 @@ unsigned shared_limit(int rows_per_thread) {
             out[r] = static_cast<unsigned>(room);
         }
         return out;
-    }();
-    return limits[static_cast<std::size_t>(rows_per_thread)];
+    })[static_cast<std::size_t>(rows_per_thread)];
 }
 
 struct Config {
