@@ -20,6 +20,7 @@
 #include "capi_internal.hpp"
 #include "common.cuh"
 #include "host/ilu_pattern.hpp"
+#include "host/per_device.hpp"
 
 #include <cuda_runtime.h>
 
@@ -251,6 +252,24 @@ __global__ void __launch_bounds__(kIluSharedThreads, 1) k_ilu_solve_shared(IluSh
     for (std::uint32_t r = threadIdx.x; r < n; r += blockDim.x) out[first + r] = xs[r];
 }
 
+// Its shared memory: the block's vector and both triangles' level starts.
+constexpr std::size_t ilu_shared_bytes(std::uint32_t rows, std::uint32_t deepest) {
+    return std::size_t(rows) * sizeof(double) + 2 * (std::size_t(deepest) + 1) * sizeof(std::uint32_t);
+}
+
+// Whether the device gives k_ilu_solve_shared the most that any factor needs: kIluSharedRows rows,
+// a level each (64 KB). Asked for once a device, and never less: the limit belongs to the kernel,
+// not to a factor.
+bool ilu_shared_opted_in() {
+    static PerDevice<bool> ready;
+    return ready.of(current_device(), [] {
+        const bool ok = cudaFuncSetAttribute(k_ilu_solve_shared, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(ilu_shared_bytes(kIluSharedRows, kIluSharedRows))) == cudaSuccess;
+        if (!ok) cudaGetLastError();
+        return ok;
+    });
+}
+
 }  // namespace
 
 // A block ILU(0) structure on the device, its values refactored per matrix.
@@ -310,12 +329,8 @@ class DeviceIlu {
             deepest_ = std::max(p.lower.deepest, p.upper.deepest);
             shared_threads_ = std::max(1u, (widest + 31) / 32) * 32;
             shared_.rows = p.rows;
-            // at most 4096 rows and so as many levels: 64 KB
-            shared_bytes_ = std::size_t(most) * sizeof(double) + 2 * (std::size_t(deepest_) + 1) * sizeof(std::uint32_t);
-            use_shared_ = shared_bytes_ <= 48 * 1024 ||
-                          cudaFuncSetAttribute(k_ilu_solve_shared, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               static_cast<int>(shared_bytes_)) == cudaSuccess;
-            cudaGetLastError();
+            shared_bytes_ = ilu_shared_bytes(most, deepest_);
+            use_shared_ = shared_bytes_ <= 48 * 1024 || ilu_shared_opted_in();
         }
     }
 

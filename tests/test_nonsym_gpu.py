@@ -295,3 +295,19 @@ def test_block_ilu_solve_shapes(planets, blocks, scale):
     got = pg.IncompleteLU(off, nb, diag, val, starts).solve(x)
     want = block_ilu_reference(off, nb, diag, val, starts, x)
     assert np.array_equal(got.view(np.int64), want.view(np.int64))
+
+
+def test_block_ilu_of_deep_blocks_beside_a_shallower_one():
+    """Tridiagonal blocks have as many levels as rows, and their level starts take the solve past
+    48 KB of shared memory: each factor keeps solving after another one of another depth is made."""
+    import planet_game_gb300 as pg
+
+    rng = np.random.default_rng(8)
+    factors = []
+    for n in (4096, 3600, 2000):
+        nb = np.array([c for r in range(n) for c in (r - 1, r + 1) if 0 <= c < n])
+        off = np.concatenate([[0], np.cumsum([(r > 0) + (r + 1 < n) for r in range(n)])])
+        diag, val, x = rng.uniform(3.0, 4.0, n), -rng.uniform(0.5, 1.0, len(nb)), rng.standard_normal(n)
+        factors.append((pg.IncompleteLU(off, nb, diag, val), x, block_ilu_reference(off, nb, diag, val, [0, n], x)))
+    for lu, x, want in factors + factors[::-1]:
+        assert np.array_equal(lu.solve(x).view(np.int64), want.view(np.int64))
