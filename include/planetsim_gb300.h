@@ -486,6 +486,7 @@ int psgb_batch_set_priority(psgb_batch* batch, int high);
  * launch shapes (tiles per thread; never change a result) and damped-Jacobi sweeps per
  * level (change the preconditioner; every tuned solve still meets the tolerance). */
 #define PSGB_MAX_LEVELS 12
+#define PSGB_COARSE_TAIL_DEFAULT PSGB_MAX_LEVELS   /* coarse_tail_level of a batch that no setting gave one */
 typedef struct psgb_tuning {
     uint32_t levels;                      /* multigrid levels of the batch */
     int pre_sweeps[PSGB_MAX_LEVELS];      /* per level, 1..8 */
@@ -497,8 +498,9 @@ typedef struct psgb_tuning {
     double tuned_solve_ms;                /* autotune: trial solve with the chosen settings */
     double default_solve_ms;              /* autotune: trial solve with the settings before */
     int trial_solves;                     /* autotune: solves timed */
-    int coarse_tail_level;                /* levels from this one down run one block per planet; 0: none
-                                             (also the default of a batch in the library's own memory) */
+    int coarse_tail_level;                /* levels from this one down run one block per planet; 0: none;
+                                             PSGB_COARSE_TAIL_DEFAULT: the library's choice, none (what an
+                                             untuned batch reports, so that its settings can be set again) */
     int block_sweeps[PSGB_MAX_LEVELS];    /* per level: Jacobi sweeps per smoothing launch, each tile in shared
                                              memory with its neighbours in other tiles held (1..8; 1 = plain) */
     int coarse_tail_single;               /* 0: a large planet's tail runs on several co-resident blocks

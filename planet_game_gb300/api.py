@@ -755,6 +755,8 @@ class Batch:
 
     @property
     def tuning(self) -> dict:
+        """The settings in use; setting them again (`set_tuning`) changes nothing. A batch that
+        no setting gave a coarse tail reports capi.COARSE_TAIL_DEFAULT as its level."""
         t = capi.Tuning()
         _raise(capi.load().psgb_batch_get_tuning(self._h, C.byref(t)))
         return _tuning_dict(t)

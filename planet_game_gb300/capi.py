@@ -59,6 +59,7 @@ class SolveOptions(C.Structure):
 
 
 MAX_LEVELS = 12
+COARSE_TAIL_DEFAULT = MAX_LEVELS   # coarse_tail_level: none set, the library chooses
 
 
 class TransportSettings(C.Structure):

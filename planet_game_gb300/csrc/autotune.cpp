@@ -108,12 +108,11 @@ void tune_shapes(Batch& b, cudaStream_t st) {
     int pick = b.tail_level;
     for (int tail = 0; tail < static_cast<int>(b.levels.size()); ++tail) {
         b.tail_level = tail;
-        b.tail_auto = tail == 0;
         const double ms = time_launches(st, [&] { vcycle<T>(b, rhs, x, kGateAlways, false, st); });
         if (best < 0.0 || ms < best) { best = ms; pick = tail; }
     }
     b.tail_level = pick;
-    b.tail_auto = pick == 0;
+    b.tail_default = false;
     PSGB_CUDA(cudaGetLastError());
 }
 
@@ -170,7 +169,7 @@ Tuning current_tuning(const Batch& b) {
     }
     t.omega = b.smoother.omega;
     t.correction = b.smoother.correction;
-    t.tail_level = b.tail_level;
+    t.tail_level = b.tail_default ? kDefaultTail : b.tail_level;
     t.tail_spread = b.tail_spread;
     t.tail_shared = b.tail_shared;
     t.tail_cluster = b.tail_cluster;
@@ -200,7 +199,7 @@ void apply_tuning(Batch& b, const Tuning& t) {
     if (!(t.omega > 0.0 && t.omega < 2.0)) throw std::invalid_argument("tuned damping must be in (0, 2)");
     if (!(t.correction > 0.0 && t.correction <= 4.0))
         throw std::invalid_argument("the coarse-grid correction scale must be in (0, 4]");
-    if (t.tail_level < 0 || static_cast<std::size_t>(t.tail_level) >= depth)
+    if (t.tail_level != kDefaultTail && (t.tail_level < 0 || static_cast<std::size_t>(t.tail_level) >= depth))
         throw std::invalid_argument("the coarse tail level must be 0 (none) or a level below the fine one");
     if (t.tail_cluster != 0 && t.tail_cluster != 2 && t.tail_cluster != 4 && t.tail_cluster != 8)
         throw std::invalid_argument("the coarse tail's cluster must be 0 (none), 2, 4 or 8 blocks");
@@ -213,8 +212,12 @@ void apply_tuning(Batch& b, const Tuning& t) {
     b.smoother.level_inner = t.inner;
     b.smoother.omega = t.omega;
     b.smoother.correction = t.correction;
-    b.tail_level = t.tail_level;
-    b.tail_auto = t.tail_level == 0;
+    if (t.tail_level == kDefaultTail) {
+        default_tail(b);
+    } else {
+        b.tail_level = t.tail_level;
+        b.tail_default = false;
+    }
     b.tail_spread = t.tail_spread;
     b.tail_shared = t.tail_shared;
     b.tail_cluster = t.tail_cluster;
@@ -372,14 +375,12 @@ Tuning autotune(Batch& b, const SolveOptions& opt, const double* rhs, const doub
                                          : tail_fits_cluster<double>(b, tail, cluster)))
                     continue;
                 b.tail_level = tail;
-                b.tail_auto = tail == 0;
                 set_mode(mode);
                 const double ms = run(best);
                 if (ms > 0.0 && ms < best_ms) { best_ms = ms; pick = tail; pick_mode = mode; }
             }
         }
         b.tail_level = pick;
-        b.tail_auto = pick == 0;
         set_mode(pick_mode);
     }
     // the fine level's tile-set sizes again, by whole solves with everything else chosen: a

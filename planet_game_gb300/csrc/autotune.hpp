@@ -4,11 +4,15 @@
 // still meet their tolerance).
 #pragma once
 
+#include "persistent.hpp"
 #include "solver.hpp"
 
 #include <vector>
 
 namespace psgb {
+
+// A tail level no batch has: none is set, the library chooses (PSGB_COARSE_TAIL_DEFAULT).
+constexpr int kDefaultTail = kMaxLevels;
 
 struct Tuning {
     std::vector<int> pre, post;                    // sweeps per level
@@ -17,7 +21,7 @@ struct Tuning {
     std::vector<std::uint8_t> sets_vector;         // per level: 1 or 4
     double omega = 0.8;
     double correction = 1.0;                       // coarse-grid correction scale
-    int tail_level = 0;                            // coarse tail from this level (0: none)
+    int tail_level = 0;                            // coarse tail from this level (0: none; kDefaultTail)
     bool tail_spread = true;                       // several blocks per large planet in the tail
     bool tail_shared = false;                      // one block per planet, the tail levels' vectors in shared memory
     unsigned tail_cluster = 0;                     // blocks of a cluster per planet (2, 4, 8; 0: none), vectors in

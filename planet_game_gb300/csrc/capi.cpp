@@ -900,6 +900,8 @@ int psgb_batch_transport_step_masked(psgb_batch* h, const uint8_t* active, const
 
 namespace {
 
+static_assert(psgb::kDefaultTail == PSGB_COARSE_TAIL_DEFAULT, "the settings' mark of the library's choice");
+
 void fill_tuning(const psgb::Tuning& t, psgb_tuning* out) {
     std::memset(out, 0, sizeof(*out));
     out->levels = static_cast<std::uint32_t>(t.pre.size());

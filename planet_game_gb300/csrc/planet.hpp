@@ -244,10 +244,8 @@ struct Batch {
     SmootherConfig smoother;
     // Levels from tail_level down run as one block per planet (coarse_tail.hpp); 0: none.
     int tail_level = 0;
-    int default_tail_level = 0;
-    // No tail asked for: a launch a phase on the coarse levels too. False: tail_level and the forms
-    // below, as a tuning with a tail level sets them.
-    bool tail_auto = true;
+    int default_tail_level = 0;        // where a tail is the default (a batch in caller's memory)
+    bool tail_default = true;          // tail_level is the library's choice, no setting
     // Several co-resident blocks per large planet in the tail (cooperative launch): per
     // tail level the packed per-block words and their count (null: one block per planet).
     bool tail_spread = true;

@@ -50,17 +50,21 @@ void upload_to(T* dst, const std::vector<T>& host) {
 
 // Tile sets pay where a level has several waves of 256-row blocks; small levels need
 // every block they can get.
+// Without a tail by default: its phases between barriers cost more than launches replayed as a
+// graph with programmatic dependent launch (a level-6 planet in FP64: 67 us a V-cycle's spread
+// tail, 5.5 ms a step with it and 2.6 without; level 8, 26.6 and 19.3 ms). A batch in caller's
+// memory records no graphs and has one.
+void default_tail(Batch& b) {
+    b.tail_default = true;
+    b.tail_level = b.store.arena() ? b.default_tail_level : 0;
+}
+
 void default_launch_shapes(Batch& b) {
     for (BatchLevel& L : b.levels) {
         L.sets_stencil = L.tiles >= kSetsMinTiles ? 2 : 1;
         L.sets_vector = L.tiles >= kSetsMinTiles ? 4 : 1;
     }
-    b.tail_level = b.default_tail_level;
-    // Without a tail by default: its phases between barriers cost more than launches replayed as a
-    // graph with programmatic dependent launch (a level-6 planet in FP64: 67 us a V-cycle's spread
-    // tail, 5.5 ms a step with it and 2.6 without; level 8, 26.6 and 19.3 ms). A batch in caller's
-    // memory records no graphs and keeps the default tail.
-    b.tail_auto = !b.store.arena();
+    default_tail(b);
 }
 
 std::unique_ptr<Planet> make_planet(std::uint32_t level, double radius_m, bool agglomerated) {
@@ -545,7 +549,7 @@ template bool tail_fits_cluster<double>(const Batch&, int, unsigned);
 
 template <typename T>
 TailForm tail_form(const Batch& b) {
-    if (b.tail_level <= 0 || b.tail_auto) return TailForm::kNone;
+    if (b.tail_level <= 0) return TailForm::kNone;
     if (b.tail_cluster != 0 && tail_fits_cluster<T>(b, b.tail_level, b.tail_cluster)) return TailForm::kCluster;
     if (b.tail_shared && tail_fits_shared<T>(b, b.tail_level)) return TailForm::kShared;
     if (b.tail_spread && b.tail_cta_at[b.tail_level] != nullptr) return TailForm::kSpread;
@@ -729,9 +733,8 @@ void vcycle(Batch& b, const T* rhs, T* x, int gate, bool first_sweep_done, cudaS
         rhs_of[l] = (l == 0) ? rhs : Pick<T>::bvec(L);
     }
     // Levels from `tail` down run in one launch (0: none).
-    const std::size_t tail = (!b.tail_auto && b.tail_level > 0 && static_cast<std::size_t>(b.tail_level) < depth)
-                                 ? static_cast<std::size_t>(b.tail_level)
-                                 : 0;
+    const std::size_t tail =
+        (b.tail_level > 0 && static_cast<std::size_t>(b.tail_level) < depth) ? static_cast<std::size_t>(b.tail_level) : 0;
     const std::size_t down_end = tail != 0 ? tail : depth - 1;
     // Planets whose only level is the fine one: dense solve there.
     if (b.dense_at[0]) launch_dense_solve<T>(dense_task<T>(b, 0, rhs, x), b.scalars, gate, st);
@@ -817,7 +820,7 @@ std::vector<int> shape_of(const Batch& b) {
         shape.push_back(b.levels[l].sets_stencil);
         shape.push_back(b.levels[l].sets_vector);
     }
-    shape.push_back(b.tail_auto ? -1 : b.tail_level);
+    shape.push_back(b.tail_level);
     shape.push_back(b.tail_spread ? 1 : 0);
     shape.push_back(b.tail_shared ? 1 : 0);
     shape.push_back(static_cast<int>(b.tail_cluster));
@@ -982,7 +985,7 @@ bool use_persistent(const Batch& b, const SolveOptions& opt) {
 // schedule's) and a batch on its caller's stream keep the kernel schedule.
 OnchipPlan* onchip_for(Batch& b, const SolveOptions& opt) {
     if (opt.schedule != kScheduleAuto || opt.method != kBiCGSTAB || b.stream == nullptr || profile_active() ||
-        !b.tail_auto)
+        b.tail_level != 0)
         return nullptr;
     OnchipPlan& plan = opt.precision == kMixed ? onchip_plan<float>(b) : onchip_plan<double>(b);
     return plan.classes.empty() ? nullptr : &plan;

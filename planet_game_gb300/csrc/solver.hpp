@@ -38,6 +38,8 @@ std::unique_ptr<Batch> make_batch_in(const std::vector<Planet*>& planets, void* 
 
 // Default tiles per thread of every level's launches (from its tile count).
 void default_launch_shapes(Batch& b);
+// The coarse tail of a batch that no setting gave one.
+void default_tail(Batch& b);
 
 // The fine-level (padded) row base of planet i inside the batch.
 inline std::int64_t fine_base(const Batch& b, std::size_t i) { return b.fine_base[i]; }

@@ -334,3 +334,56 @@ def test_vector_launches_of_large_levels(meshes, precision):
         small, small_reports = run(inputs[k:k + 1], 1)
         assert np.array_equal(out[k], small[0]) and np.array_equal(four[k], small[0])
         assert reports[k].iterations == small_reports[0].iterations
+
+
+# the second and third on thread-block clusters untuned; L2 has no level for a tail
+@pytest.mark.parametrize("levels,precision", [((6,), "fp64"), ((4,), "fp64"), ((5, 3, 4), "mixed"), ((7, 5), "mixed"),
+                                              ((2,), "fp64")])
+def test_settings_read_back_and_set_again_change_nothing(meshes, levels, precision):
+    """Results, counts, settings and the solve's launches, of a fresh batch, with a tail set, and
+    after clearing it; and of a planet's own solves."""
+    import planet_game_gb300 as pg
+    from planet_game_gb300 import capi, workloads as W
+
+    ms = [meshes(l, 4.0e6 + 3e5 * i) for i, l in enumerate(levels)]
+    inputs = [W.step_inputs(m, seed=60 + i) for i, m in enumerate(ms)]
+
+    def run(step):
+        step()   # graphs, plans
+        before = capi.load().psgb_launch_count()
+        out, reports = step()
+        return out, [(r.status, r.iterations, r.refinements) for r in reports], capi.load().psgb_launch_count() - before
+
+    def same(a, b):
+        assert a[1:] == b[1:] and all(np.array_equal(x, y) for x, y in zip(a[0], b[0]))
+
+    batch = pg.Batch(ms)
+    step = lambda: batch.transport_step([i.t0 for i in inputs], [i.source for i in inputs], 4e7, inputs[0].dt,
+                                        conductance=[4e13] * len(ms), precision=precision)
+    fresh, settings = run(step), batch.tuning
+    batch.set_tuning(settings)
+    assert batch.tuning == settings
+    same(run(step), fresh)
+    if settings["levels"] > 1:
+        tail = dict(settings, coarse_tail_level=1, coarse_tail_single=1)
+        batch.set_tuning(tail)
+        with_tail, reported = run(step), batch.tuning
+        assert reported["coarse_tail_level"] == 1 and reported["coarse_tail_blocks"] == len(ms)
+        assert with_tail[2] != fresh[2]
+        batch.set_tuning(reported)
+        same(run(step), with_tail)
+        assert batch.tuning == reported
+        batch.set_tuning(None)
+        same(run(step), fresh)
+        bad = dict(settings, coarse_tail_level=settings["levels"])
+        with pytest.raises(ValueError, match="coarse tail level"):
+            batch.set_tuning(bad)
+
+    m, inp = ms[0], inputs[0]
+    m.set_tuning(None)
+    alone = lambda: (lambda t, _, r: ([t], [r]))(*pg.transport_step(m, inp.t0, inp.source, 4e7, inp.dt, 4e13,
+                                                                    precision=precision))
+    fresh = run(alone)
+    m.set_tuning(m.tuning)
+    same(run(alone), fresh)
+    m.set_tuning(None)
