@@ -492,8 +492,7 @@ typedef struct psgb_tuning {
     int pre_sweeps[PSGB_MAX_LEVELS];      /* per level, 1..8 */
     int post_sweeps[PSGB_MAX_LEVELS];     /* per level, 0..8 */
     int stencil_tiles[PSGB_MAX_LEVELS];   /* tiles per thread of the stencil launches: 1 or 2 */
-    int vector_tiles[PSGB_MAX_LEVELS];    /* tiles per thread of the vector launches: 1 or 4
-                                             (levels of 2,432 tiles and more run 4 whichever) */
+    int vector_tiles[PSGB_MAX_LEVELS];    /* tiles per thread of the vector launches: 1 or 4 */
     double jacobi_omega;
     double tuned_solve_ms;                /* autotune: trial solve with the chosen settings */
     double default_solve_ms;              /* autotune: trial solve with the settings before */

@@ -90,8 +90,6 @@ void tune_shapes(Batch& b, cudaStream_t st) {
         }
         L.sets_stencil = pick;
         if (l != 0) continue;
-        L.sets_vector = 4;
-        if (L.tiles >= kSetsMinTiles) continue;   // the one shape it runs
         pick = 1;
         for (std::uint8_t sets : {std::uint8_t(1), std::uint8_t(4)}) {
             L.sets_vector = sets;
@@ -393,7 +391,7 @@ Tuning autotune(Batch& b, const SolveOptions& opt, const double* rhs, const doub
         std::uint8_t ps = s0, pv = v0;
         for (std::uint8_t s : {std::uint8_t(1), std::uint8_t(2)}) {
             for (std::uint8_t v : {std::uint8_t(1), std::uint8_t(4)}) {
-                if ((s == s0 && v == v0) || (v == 1 && F.tiles >= kSetsMinTiles)) continue;
+                if (s == s0 && v == v0) continue;
                 F.sets_stencil = s;
                 F.sets_vector = v;
                 const double ms = run(best);

@@ -222,19 +222,6 @@ struct SmootherConfig {
     bool starts_in_x(std::size_t l) const { return ((pre_at(l) - 1 + post_at(l)) % 2) == 0; }
 };
 
-// Levels with at least this many tiles (two waves of eight 256-thread blocks on 152 SMs)
-// use multi-tile sets by default.
-constexpr std::uint32_t kSetsMinTiles = 2 * 8 * 152;
-
-// Tiles a thread of the level's vector launches: what is set, but four on those levels. A block a
-// tile was the better shape there while one lane added up all sums of a block; since each sum has a
-// lane, four L7 planets (2,564 tiles) solve in 6.90 ms with four tiles against 7.02 with one, 16 L6
-// planets 4.14 and 4.25, the lanes of the 64-planet mix 10.96 and 11.75; two L7 planets (1,282
-// tiles) 5.75 and 5.74, one 4.38 and 4.26. The bits are the same.
-inline std::uint8_t vector_sets(const BatchLevel& level) {
-    return level.tiles >= kSetsMinTiles ? std::uint8_t(4) : level.sets_vector;
-}
-
 struct Batch {
     std::vector<Planet*> planets;
     std::uint32_t instances = 0;

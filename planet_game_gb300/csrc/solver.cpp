@@ -38,6 +38,13 @@ Batch::~Batch() {
 
 namespace {
 
+// Levels with at least this many tiles (two waves of eight 256-thread blocks on 152 SMs)
+// use multi-tile sets by default: four L7 planets (2,564 tiles) solve in 6.90 ms with four tiles
+// a thread of the vector launches against 7.02 with one, 16 L6 planets in 4.14 against 4.25, the
+// lanes of the 64-planet mix in 10.96 against 11.75; two L7 planets (1,282 tiles) in 5.75 and
+// 5.74, one in 4.38 and 4.26. The bits are the same; a setting of either is what runs.
+constexpr std::uint32_t kSetsMinTiles = 2 * 8 * 152;
+
 // Levels whose planets hold at most this many rows each run in the coarse tail.
 constexpr std::uint32_t kTailRows = 4096;
 
@@ -510,7 +517,7 @@ static LevelView<T> make_view(const BatchLevel& L, const T* vd, const T* inv, st
     LevelView<T> v{L.rows,         L.width,        L.tiles,      L.col,
                    vd,             inv,            L.tile_inst,  L.tile_rows,
                    L.tile_sweep,   L.tile_meta,    nullptr,
-                   L.sets_stencil, vector_sets(L), static_cast<std::uint8_t>(level)};
+                   L.sets_stencil, L.sets_vector,  static_cast<std::uint8_t>(level)};
     v.scol = L.scol;
     v.tile_shift = L.tile_shift;
     v.spitch = L.spitch;
