@@ -454,6 +454,7 @@ PROFILED_FAMILIES = (
     ("krylov_vector", "k_bicg_init / p / s / x (vector updates with fused dots)"),
     ("refine", "k_outer_init / residual / update (FP64 refinement)"),
     ("step", "k_step_rhs / k_step_finish (right-hand side, flux form, closure sums)"),
+    ("onchip", "k_onchip_solve (whole solves of small planets; no bytes counted)"),
 )
 
 

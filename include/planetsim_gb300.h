@@ -554,8 +554,12 @@ int psgb_column_radiation(uint32_t cells, uint32_t layers, const psgb_column_con
 /* ---- launch accounting and kernel timing (no counterpart in the reference) -------
  * psgb_launch_count: kernels this library has launched since it was loaded.
  * psgb_profile_begin: from now on, time every launch of one kernel family ("smooth",
- * "residual", "restrict", "prolong", "dense", "krylov_spmv", "krylov_vector", "refine",
- * "setup", "step", "operator", "column") with CUDA events on its launching stream.
+ * "residual", "restrict", "prolong", their coarse levels' "smooth_coarse",
+ * "residual_coarse", "restrict_coarse", "prolong_coarse", "dense", "krylov_spmv",
+ * "krylov_vector", "refine", "persistent", "onchip", "setup", "step", "operator",
+ * "column") with CUDA events on its launching stream. The calls run as they do without a
+ * profile, but that the kernel schedule launches its kernels one by one, not as graphs;
+ * planets solved on chip launch "onchip" alone (PSGB_SCHEDULE_KERNELS has the others).
  * psgb_profile_end: synchronises, returns the summed device time (ms) and launch count of
  * that family, and the algorithmic bytes the Jacobi sweeps moved since the profile began. */
 uint64_t psgb_launch_count(void);

@@ -1063,7 +1063,7 @@ void onchip_launch(const OnchipArgs<T>& args, int rows_per_thread, unsigned thre
     if (shared_bytes > oc::shared_limit<T>(rows_per_thread)) throw std::logic_error("on-chip solve: the planet does not fit");
     const unsigned cluster = static_cast<unsigned>(args.cluster);
     oc::Config c(cluster, args.planets * cluster, threads, shared_bytes, st);
-    PSGB_LAUNCH(kFamPersistent, st, {
+    PSGB_LAUNCH(kFamOnchip, st, {
         const cudaError_t e = cudaLaunchKernelEx(&c.cfg, oc::kernel_of<T>(rows_per_thread), args);
         if (e != cudaSuccess) throw std::runtime_error(std::string("on-chip solve launch: ") + cudaGetErrorString(e));
     });

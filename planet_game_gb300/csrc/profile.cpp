@@ -37,7 +37,7 @@ constexpr std::size_t kMaxEvents = 1 << 16;
 const char* const kNames[kFamCount] = {"smooth", "residual", "restrict", "prolong", "dense", "krylov_spmv",
                                        "krylov_vector", "refine", "setup", "step", "operator", "column",
                                        "persistent", "smooth_coarse", "residual_coarse", "restrict_coarse",
-                                       "prolong_coarse"};
+                                       "prolong_coarse", "onchip"};
 
 }  // namespace
 

@@ -30,6 +30,8 @@ enum KernelFamily : int {
     kFamResidualCoarse,  // V-cycle residual of the coarse levels
     kFamRestrictCoarse,  // restriction onto a level below the first coarse one
     kFamProlongCoarse,   // prolongation onto a coarse level
+    kFamOnchip,          // whole solves on thread-block clusters (a launch a planet shape; no bytes counted:
+                         // their vectors stay in shared memory)
     kFamCount
 };
 

@@ -988,11 +988,9 @@ bool use_persistent(const Batch& b, const SolveOptions& opt) {
 }
 
 // The on-chip solves of the automatic schedule: BiCGSTAB on planets that fit a cluster. A
-// tuning that asks for a coarse tail, a recording profile (whose families are the kernel
-// schedule's) and a batch on its caller's stream keep the kernel schedule.
+// tuning that asks for a coarse tail and a batch on its caller's stream keep the kernel schedule.
 OnchipPlan* onchip_for(Batch& b, const SolveOptions& opt) {
-    if (opt.schedule != kScheduleAuto || opt.method != kBiCGSTAB || b.stream == nullptr || profile_active() ||
-        b.tail_level != 0)
+    if (opt.schedule != kScheduleAuto || opt.method != kBiCGSTAB || b.stream == nullptr || b.tail_level != 0)
         return nullptr;
     OnchipPlan& plan = opt.precision == kMixed ? onchip_plan<float>(b) : onchip_plan<double>(b);
     return plan.classes.empty() ? nullptr : &plan;

@@ -93,3 +93,39 @@ def test_non_finite_source_reports_and_keeps_the_other_planets(meshes):
     with pytest.raises(Exception, match="non-finite"):
         batch.transport_step(*args(bad), edge_conductance=edges, precision="mixed")
     same(good, batch.transport_step(*args(inputs[0].source), edge_conductance=edges, precision="mixed"))
+
+
+def launches_of(family, call):
+    """The launches of a kernel family during a call, and the call's result."""
+    import ctypes as C
+
+    from planet_game_gb300 import capi
+
+    lib = capi.load()
+    ms, count, swept = C.c_double(), C.c_uint64(), C.c_uint64()
+    capi.check(lib.psgb_profile_begin(family.encode()))
+    try:
+        out = call()
+    finally:
+        capi.check(lib.psgb_profile_end(C.byref(ms), C.byref(count), C.byref(swept)))
+    assert (ms.value > 0.0) == (count.value > 0)
+    return count.value, out
+
+
+@pytest.mark.parametrize("levels,precision", [((4,), "fp64"), ((5, 3, 4, 5), "mixed")])
+def test_a_recording_profile_times_the_solves_that_run_without_it(meshes, levels, precision):
+    import planet_game_gb300 as pg
+
+    ms = [meshes(l, 3.3e6 + 2e5 * i) for i, l in enumerate(levels)]
+    batch, inputs = pg.Batch(ms), [inputs_of(m, 60 + i) for i, m in enumerate(ms)]
+    plain = step(batch, inputs, precision=precision)
+    for schedule in ("auto", "kernels"):
+        call = lambda: step(batch, inputs, precision=precision, schedule=schedule)
+        onchip, recorded = launches_of("onchip", call)
+        smooth, again = launches_of("smooth", call)
+        same(plain, recorded)
+        same(plain, again)
+        if schedule == "auto":   # a launch a planet shape, no sweep of the kernel schedule
+            assert onchip == len(set(levels)) and smooth == 0
+        else:
+            assert onchip == 0 and smooth > 0
