@@ -129,3 +129,73 @@ def test_a_recording_profile_times_the_solves_that_run_without_it(meshes, levels
             assert onchip == len(set(levels)) and smooth == 0
         else:
             assert onchip == 0 and smooth > 0
+
+
+# every form of the kernel that a batch's planets take: rows a thread, with block-local coarse
+# sweeps and a scaled correction too, and batches that keep the kernel schedule
+@pytest.mark.parametrize("precision,levels,onchip", [("fp64", (4,), True), ("fp64", (5,), True), ("fp64", (5, 4, 5, 3), True),
+                                                     ("fp64", (6,), False), ("mixed", (5,), True), ("mixed", (6,), True),
+                                                     ("mixed", (5, 6, 4, 5, 3), True), ("mixed", (5, 7), False)])
+def test_which_batches_go_on_chip(meshes, precision, levels, onchip):
+    """Tuned and untuned: that the path is the one meant, and the kernel schedule's bits."""
+    import planet_game_gb300 as pg
+
+    ms = [meshes(l, 3.1e6 + 3e5 * i) for i, l in enumerate(levels)]
+    inputs = [inputs_of(m, 80 + i) for i, m in enumerate(ms)]
+    batch = pg.Batch(ms)
+    depth = batch.tuning["levels"]
+    for inner, correction, omega in ((0, 1.0, 0.8), (6, 1.0, 1.0), (3, 2.0, 0.9), (1, 1.5, 0.8)):
+        if inner:
+            batch.set_tuning({"pre_sweeps": [1] + [2] * (depth - 1), "post_sweeps": [1] + [2] * (depth - 1),
+                              "stencil_tiles": [1] * depth, "vector_tiles": [1] * depth,
+                              "block_sweeps": [1] + [inner] * (depth - 1), "jacobi_omega": omega,
+                              "coarse_correction": correction})
+        count, got = launches_of("onchip", lambda: step(batch, inputs, precision=precision))
+        assert count == (len(set(levels)) if onchip else 0)
+        same(got, step(batch, inputs, precision=precision, schedule="kernels"))
+
+
+def test_priority_and_masks_change_nothing(meshes):
+    """After a solve, set_priority drops the plans with their streams; a changing mask keeps them."""
+    import planet_game_gb300 as pg
+
+    ms = [meshes(l, 3.0e6 + 2e5 * i) for i, l in enumerate((5, 3, 4, 5, 4))]
+    inputs = [inputs_of(m, 100 + i) for i, m in enumerate(ms)]
+    batch = pg.Batch(ms)
+    masks = (range(5), (0, 2), (4,), (1, 3), range(5))
+    want = [step(batch, inputs, precision="mixed", keep=keep, schedule="kernels") for keep in masks]
+    for high in (None, True, False):
+        if high is not None:
+            batch.set_priority(high)
+        for keep, ref in zip(masks, want):
+            count, got = launches_of("onchip", lambda: step(batch, inputs, precision="mixed", keep=keep))
+            assert count == 3
+            same(got, ref)
+
+
+def test_batches_side_by_side(meshes):
+    """Two batches solved on chip from two threads, beside one on the kernel schedule."""
+    import threading
+
+    import planet_game_gb300 as pg
+
+    jobs = []
+    for k, (levels, precision) in enumerate((((5, 4, 3), "mixed"), ((4, 5), "fp64"), ((7,), "mixed"))):
+        ms = [meshes(l, 3.0e6 + 2e5 * i + 1e5 * k) for i, l in enumerate(levels)]
+        inputs = [inputs_of(m, 120 + 10 * k + i) for i, m in enumerate(ms)]
+        batch = pg.Batch(ms)
+        jobs.append((batch, inputs, precision, step(batch, inputs, precision=precision, schedule="kernels"), []))
+
+    def work(batch, inputs, precision, _, out):
+        for _ in range(5):
+            out.append(step(batch, inputs, precision=precision))
+
+    threads = [threading.Thread(target=work, args=job) for job in jobs]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for *_, want, got in jobs:
+        assert len(got) == 5
+        for g in got:
+            same(g, want)
