@@ -173,17 +173,10 @@ void choose(const Batch& b, OnchipClass& c) {
 
 }  // namespace
 
+namespace {
+
 template <typename T>
-OnchipPlan& onchip_plan(Batch& b) {
-    // the smoother decides how rows are shared out (block-local sweeps) and how many phases
-    // a V-cycle has
-    std::vector<int> key{static_cast<int>(sizeof(T))};
-    for (std::size_t l = 0; l < b.levels.size(); ++l) {
-        key.push_back(b.smoother.inner_at(l) > 1 ? 1 : 0);
-        key.push_back(b.smoother.pre_at(l) + b.smoother.post_at(l));
-    }
-    std::unique_ptr<OnchipPlan>& slot = b.onchip[key];
-    if (slot) return *slot;
+std::unique_ptr<OnchipPlan> make_plan(const Batch& b) {
     auto plan = std::make_unique<OnchipPlan>();
     std::map<std::vector<std::uint32_t>, OnchipClass> classes;
     for (std::uint32_t i = 0; i < b.instances; ++i) {
@@ -231,11 +224,8 @@ OnchipPlan& onchip_plan(Batch& b) {
         plan->done.push_back(e);
         if (plan->fork == nullptr) PSGB_CUDA(cudaEventCreateWithFlags(&plan->fork, cudaEventDisableTiming));
     }
-    slot = std::move(plan);
-    return *slot;
+    return plan;
 }
-
-namespace {
 
 template <typename T>
 OnchipArgs<T> arguments(Batch& b, const OnchipClass& c) {
@@ -276,6 +266,18 @@ OnchipArgs<T> arguments(Batch& b, const OnchipClass& c) {
 }
 
 }  // namespace
+
+template <typename T>
+OnchipPlan& onchip_plan(Batch& b) {
+    // the smoother decides how rows are shared out (block-local sweeps) and how many phases
+    // a V-cycle has
+    std::vector<int> key{static_cast<int>(sizeof(T))};
+    for (std::size_t l = 0; l < b.levels.size(); ++l) {
+        key.push_back(b.smoother.inner_at(l) > 1 ? 1 : 0);
+        key.push_back(b.smoother.pre_at(l) + b.smoother.post_at(l));
+    }
+    return *b.onchip.of(key, [&] { return make_plan<T>(b); });
+}
 
 template <typename T>
 void onchip_solve(Batch& b, OnchipPlan& plan, const SolveOptions& opt, const double* rhs, double* x, double inner_tol,

@@ -36,7 +36,7 @@ struct OnchipPlan {
     cudaEvent_t fork = nullptr;
 };
 
-// The plan of a batch in precision T under its present smoother (kept with the batch).
+// The plan of a batch in precision T under its present smoother (the batch keeps its last few).
 template <typename T>
 OnchipPlan& onchip_plan(Batch& b);
 

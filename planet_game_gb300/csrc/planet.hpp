@@ -9,6 +9,7 @@
 #pragma once
 
 #include "host/hierarchy.hpp"
+#include "host/kept_few.hpp"
 #include "host/mesh.hpp"
 #include "kernels.hpp"
 
@@ -281,8 +282,9 @@ struct Batch {
     cudaEvent_t fence_in = nullptr, fence_out = nullptr;
     std::map<GraphKey, GraphEntry> graphs;
     bool use_graphs = true;
-    // on-chip solves: per precision and block-local levels, which planets and how
-    std::map<std::vector<int>, std::unique_ptr<OnchipPlan>> onchip;
+    // on-chip solves: per precision, sweeps and block-local levels, which planets and how. A plan
+    // holds streams and device lists, and a tuner goes through dozens of sweeps: the last few stay.
+    KeptFew<std::vector<int>, std::unique_ptr<OnchipPlan>, 4> onchip;
     // transport-step buffers (fine layout)
     double* slope_of = nullptr;        // [instances] dt / C
     double* t0 = nullptr;              // [P0]

@@ -199,3 +199,18 @@ def test_batches_side_by_side(meshes):
         assert len(got) == 5
         for g in got:
             same(g, want)
+
+
+def test_more_sweep_settings_than_plans_are_kept(meshes):
+    import planet_game_gb300 as pg
+
+    ms = [meshes(l, 3.2e6 + 2e5 * i) for i, l in enumerate((4, 5, 3))]
+    inputs = [inputs_of(m, 150 + i) for i, m in enumerate(ms)]
+    batch = pg.Batch(ms)
+    settings = [dict(pre_sweeps=a, post_sweeps=b, precision=p) for p in ("mixed", "fp64") for a, b in ((1, 0), (1, 1), (2, 1), (3, 3))]
+    want = [step(batch, inputs, schedule="kernels", **s) for s in settings]
+    for _ in range(2):
+        for s, ref in zip(settings, want):
+            count, got = launches_of("onchip", lambda: step(batch, inputs, **s))
+            assert count == 3
+            same(got, ref)
