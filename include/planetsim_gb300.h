@@ -93,7 +93,9 @@ typedef struct psgb_planet_info {
     uint64_t cells, edges, directed_edges, corners;
     uint32_t levels;             /* multigrid levels (the last one is solved densely) */
     uint32_t level_rows[8];      /* rows per multigrid level */
-    uint64_t device_bytes;       /* HBM held by the planet (mesh + its solo batch) */
+    uint64_t device_bytes;       /* HBM held by the planet: mesh, its solo batch, and what its
+                                    other solves keep between calls (a tracer solve's vectors
+                                    stay for each layer count) */
     uint64_t fine_cells;         /* agglomerated planets: cells of the fine mesh; 0 otherwise */
 } psgb_planet_info;
 int psgb_planet_info_get(const psgb_planet* planet, psgb_planet_info* out);

@@ -380,7 +380,9 @@ int psgb_planet_info_get(const psgb_planet* h, psgb_planet_info* out) {
         out->corners = p.mesh.corners;
         out->levels = static_cast<uint32_t>(p.hierarchy.levels.size());
         for (std::size_t l = 0; l < p.hierarchy.levels.size() && l < 8; ++l) out->level_rows[l] = p.hierarchy.levels[l].size;
-        out->device_bytes = p.store.bytes() + (p.solo ? p.solo->store.bytes() : 0) + h->stage_store.bytes();
+        out->device_bytes = p.store.bytes() + (p.solo ? p.solo->store.bytes() : 0) + h->stage_store.bytes() +
+                            h->newton_store.bytes() + (h->nonsym ? psgb::device_bytes(*h->nonsym) : 0) +
+                            (h->multi ? h->multi->store.bytes() : 0);
         out->fine_cells = p.group_of_cell.size();
         return PSGB_OK;
     });

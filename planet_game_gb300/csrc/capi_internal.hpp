@@ -15,6 +15,7 @@
 namespace psgb {
 
 struct NonsymContext;   // the non-symmetric solves' per-planet structures (nonsym.cu)
+std::size_t device_bytes(const NonsymContext& context);
 
 // A numerical breakdown reported as PSGB_ERR_BREAKDOWN (a zero ILU pivot).
 struct Breakdown : std::runtime_error {

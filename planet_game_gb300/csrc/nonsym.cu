@@ -365,6 +365,7 @@ class DeviceIlu {
     }
 
     std::uint32_t rows() const { return rows_; }
+    std::size_t device_bytes() const { return store_.bytes(); }
 
   private:
     DeviceStore store_;
@@ -1064,10 +1065,18 @@ struct NonsymContext {
         Stacked view{};
         Ell ell{};
         std::unique_ptr<DeviceIlu> ilu;
-        std::unique_ptr<struct TracerWork> work;   // on the first solve
+        std::unique_ptr<TracerWork> work;   // on the first solve
     };
     std::map<std::uint32_t, std::unique_ptr<StackedSystem>> stacked;
 };
+
+std::size_t device_bytes(const NonsymContext& c) {
+    std::size_t bytes = c.store.bytes() + (c.graph_ilu ? c.graph_ilu->device_bytes() : 0);
+    for (const auto& [layers, s] : c.stacked) {
+        bytes += s->store.bytes() + (s->ilu ? s->ilu->device_bytes() : 0) + (s->work ? s->work->store.bytes() : 0);
+    }
+    return bytes;
+}
 
 namespace {
 

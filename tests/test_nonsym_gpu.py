@@ -311,3 +311,27 @@ def test_block_ilu_of_deep_blocks_beside_a_shallower_one():
         factors.append((pg.IncompleteLU(off, nb, diag, val), x, block_ilu_reference(off, nb, diag, val, [0, n], x)))
     for lu, x, want in factors + factors[::-1]:
         assert np.array_equal(lu.solve(x).view(np.int64), want.view(np.int64))
+
+
+def test_the_tracer_solves_memory_is_counted():
+    """What a planet's tracer solves keep between calls is part of its device bytes: the vectors of
+    each layer count, once."""
+    import planet_game_gb300 as pg
+    from planet_game_gb300 import workloads as W
+
+    p = pg.make_icosphere(4, RADIUS)
+    g = pg.mesh_transport_graph(p)
+    solved = {}
+    for layers in (2, 3, 2, 3):
+        flux = W.antisymmetric_layer_fluxes(g.offset, g.neighbour, layers, 2e9, seed=7, column_balanced=True)
+        before = p.device_bytes()
+        pg.solve_implicit_tracer(p, pg.AdvectionDiffusion(layers, np.full(len(g.neighbour), 2e8), flux, CP),
+                                 g.area_m2 * 100000.0 / (9.81 * layers), W.tracer_field(layers * p.cell_count, seed=8),
+                                 2.63e6)
+        grown = p.device_bytes() - before
+        if layers in solved:
+            assert grown == 0
+        else:   # sixteen vectors of the stacked rows and the off-diagonals twice at least
+            rows, entries = layers * p.cell_count, layers * len(g.neighbour)
+            assert grown >= 8 * (16 * rows + 2 * entries)
+        solved[layers] = grown
