@@ -237,6 +237,9 @@ typedef struct psgb_step_params {
                                        psgb_batch_set_edge_conductance (edge_conductance NULL) */
 } psgb_step_params;
 
+/* The sums are formed in a fixed tree: over each 256-cell tile, then over every 32nd tile in
+ * order, then those 32 in pairs (not tile by tile). The same inputs give the same bits, alone or
+ * in a batch. */
 typedef struct psgb_step_report {
     psgb_solve_report solve;
     double sum_W;                /* sum A H (zero to rounding) */
@@ -594,7 +597,10 @@ typedef struct psgb_server psgb_server;
 
 typedef struct psgb_server_config {
     double budget_bytes;          /* device memory for resident lanes */
-    double bytes_per_cell;        /* a resident lane's estimate per cell (<= 0: 700) */
+    double bytes_per_cell;        /* a resident lane's estimate per cell (<= 0: 700): its batch (682 at
+                                     level 3, 661 at 4, 511 at 5, 492 to 503 from 6 up) and 16 of state.
+                                     The planets' meshes, uploaded once and kept for the server's life
+                                     (346 to 409), are not part of it */
     psgb_solve_options options;   /* every step's solve */
     int autotune;                 /* nonzero: tune each lane at its first admission (psgb_batch_autotune),
                                      reapplied at later admissions */

@@ -19,7 +19,7 @@ namespace psgb {
 constexpr unsigned kOnchipRankShift = 12;
 constexpr unsigned kOnchipMaxSpan = 1u << kOnchipRankShift;
 constexpr unsigned kOnchipMaxCluster = 16;
-constexpr unsigned kOnchipMaxTiles = 256;   // fine-level tiles of a planet (one thread sums each)
+constexpr unsigned kOnchipMaxTiles = 256;   // fine-level tiles of a planet (a reduction sums eight sets of 32, a lane a tile)
 
 template <typename T>
 struct OnchipLevel {
@@ -77,8 +77,6 @@ constexpr int kOnchipMaxPhases = 256;
 constexpr unsigned kOnchipPhaseBytes = 48;
 template <typename T>
 int onchip_active_clusters(int rows_per_thread, unsigned cluster, unsigned threads, std::size_t shared_bytes);
-template <typename T>
-unsigned onchip_max_threads(int rows_per_thread);
 template <typename T>
 void onchip_launch(const OnchipArgs<T>& args, int rows_per_thread, unsigned threads, std::size_t shared_bytes,
                    cudaStream_t st);

@@ -856,9 +856,12 @@ struct Solve {
 };
 
 // At most kOnchipThreads threads a block. Few threads with several rows each: the cluster
-// barrier is cheaper (0.19 us with 256 threads, 0.29 with 1024), and the whole solve, its rows'
-// matrix and addresses with it, stays in registers, where 1024 threads would spill to an L1 that
-// the shared memory leaves no room in.
+// barrier is cheaper (0.19 us with 256 threads, 0.29 with 1024), and a thread has 168 registers
+// for the solve, its rows' matrix and addresses with it, where 1024 threads have 64 and spill
+// most of it to an L1 that the shared memory leaves no room in. FP32 with one or two rows a thread
+// stays in registers whole; the others spill a little (bytes of stores and loads a thread: FP32
+// four rows 168 and 188, seven 12 and 24; FP64 one row 44 and 64, two 388 and 420, four 172 and
+// 216).
 template <typename T, int R>
 __global__ void __launch_bounds__(kOnchipThreads, 1) k_onchip_solve(const __grid_constant__ OnchipArgs<T> a) {
     extern __shared__ __align__(16) unsigned char onchip_smem[];

@@ -192,7 +192,7 @@ __global__ void k_step_rhs(std::uint32_t rows, const std::int32_t* __restrict__ 
 
 // Flux form of the solved temperature: H = (1/A) sum_k G_k w_k (T_k - T_c), with G
 // the planet's K or the per-entry conductance; T_new = T0 + s (S + H). Per-tile
-// partial sums, then per-planet sums in tile order: sum A H, sum A |H|, sum A H T,
+// partial sums, then per-planet sums in k_sum_tiles' tree: sum A H, sum A |H|, sum A H T,
 // sum A S, sum A |S|, sum A (T_new - T0) / s.
 __global__ void k_step_finish(std::uint32_t P, const std::int32_t* __restrict__ tile_inst,
                               const std::int32_t* __restrict__ tile_rows,
